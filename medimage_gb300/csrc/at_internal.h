@@ -45,6 +45,42 @@ struct __align__(16) RayHdr {
 };
 static_assert(sizeof(RayHdr) == 32, "RayHdr must stay 32 bytes");
 
+// A ray as a straight line through the grid, for the projectors that step row
+// by row instead of segment by segment (fan / ray plans, Plan::line_ok).  Rows
+// count along the axis the ray runs closer to (x, or y when kLineSwap is set),
+// columns along the other, so a row holds at most one column crossing.  Rows
+// are walked in the order in which the columns increase: upwards, or downwards
+// (kLineDown), when row u is step n-1-u.  Row coordinates run along the walk,
+// relative to n/2.  The crossing from column c0 + k into the next is at
+// fmaf(kv0 + k, inv, e_ref), for every k: e_ref belongs to a crossing near the
+// ray's middle, so the products stay small.  A row's part before the crossing,
+// times len, is the segment in the current column, the rest of the row the
+// segment in the next one.
+struct __align__(16) LineRay {
+  float e_ref, inv, kv0, len;  // len: mm per row
+  int32_t off;     // column c0 of row 0 of the ray's copy, among the padded image copies (line_pitch)
+  uint32_t rows;   // first step | last step << 16, a row around those in which it meets the grid;
+                   // first > last: no line
+  int32_t corr0;   // first correction (LineCorr), flags' upper bits: how many
+  uint32_t flags;  // kLineSwap | kLineDown | corrections << 8
+};
+static_assert(sizeof(LineRay) == 32, "LineRay must stay 32 bytes");
+constexpr uint32_t kLineSwap = 1u;  // rows count along y
+constexpr uint32_t kLineDown = 2u;  // rows are walked from n-1 down
+// What the traversal has and the line does not, as (pixel, weight) to add:
+// minus the last piece of a ray that the reference's loop leaves out
+// (tracing.cpp:118), or all segments of a ray that no line describes.
+struct LineCorr {
+  int32_t pix;  // x*n + y, | kCorrForwardOnly for a segment off the grid
+  float w;      // mm
+};
+constexpr int32_t kCorrForwardOnly = 1 << 30;
+// The padded image copies those walks read: rows of line_pitch(n) elements,
+// column c at c + kLinePad, zeros around the columns, n rows row-major then n
+// rows transposed.  A walk strays at most two columns past the grid.
+constexpr int kLinePad = 4;
+constexpr int line_pitch(int n) { return (n + 2 * kLinePad + 3) & ~3; }
+
 struct GcSeg {   // one GoldenC walk segment
   int32_t pix;   // Y*512 + X (tile-global, symmetry 0 frame)
   float w;
@@ -103,6 +139,13 @@ struct Plan {
   uint32_t *blk_word_d = nullptr;
   uint8_t *blk_off_d = nullptr;
   int nblocks_per_view = 0, nblocks = 0;
+  // every ray as a line (LineRay), with corrections where the traversal departs
+  // from it; not built (line_ok = 0) for the plain FP32 traversal, and for ray
+  // tables most of whose rays are no lines through the whole grid
+  int line_ok = 0;
+  LineRay *line_d = nullptr;
+  LineCorr *lcorr_d = nullptr;
+  int64_t ncorr = 0;
   // back projection: one entry per (ray, 16x16 tile) run of the traversal,
   // grouped by tile, longest runs first.  Entry = {ray, k_in | nk << 14 |
   // cx_in << 19, the run's decision bits (bit j = segment k_in + j; a run in a

@@ -1,0 +1,163 @@
+// line.cuh -- the row-by-row walk of a ray's line (LineRay), shared by the
+// forward projectors that gather through L1 (project.cu) and from shared
+// memory (slab.cu).  Both run exactly these operations per row and fold the
+// row sums at the same rows, so their sums agree bit for bit.
+#pragma once
+
+#include "epilogue.cuh"
+
+namespace medimg {
+
+// one pixel of G scans projected together (three scans take the float4 form)
+template <int G>
+struct Elem;
+template <>
+struct Elem<1> {
+  using T = float;
+};
+template <>
+struct Elem<2> {
+  using T = float2;
+};
+template <>
+struct Elem<4> {
+  using T = float4;
+};
+
+// two fmaf side by side in one instruction (the same rounding)
+__device__ __forceinline__ void fma_pair(float &x, float &y, float w, float a, float b) {
+  uint64_t s, v, ww;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(s) : "f"(x), "f"(y));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
+  asm("mov.b64 %0, {%1, %1};" : "=l"(ww) : "f"(w));
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(s) : "l"(ww), "l"(v));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(s));
+}
+
+template <int G>
+__device__ __forceinline__ void fma_elem(float (&part)[G], float wt, const typename Elem<G>::T &v) {
+  if constexpr (G == 1) {
+    part[0] = fmaf(wt, v, part[0]);
+  } else if constexpr (G == 2) {
+    fma_pair(part[0], part[1], wt, v.x, v.y);
+  } else {
+    fma_pair(part[0], part[1], wt, v.x, v.y);
+    fma_pair(part[2], part[3], wt, v.z, v.w);
+  }
+}
+
+template <int G>
+__device__ __forceinline__ typename Elem<G>::T zero_elem() {
+  if constexpr (G == 1) return 0.f;
+  else if constexpr (G == 2) return make_float2(0.f, 0.f);
+  else return make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
+// A ray's walk over the rows of its copy, in blocks of 32 steps (steps 0..31 of
+// the copy, 32..63, ...), with row coordinates relative to the block's middle.  A block's state depends on the ray and the block
+// alone (enter()), and the block sums are folded in order into a Kahan total
+// (LineTotal), so a ray's blocks may be walked by one thread after another or
+// by several threads: the sums are the same bit for bit.
+template <int G>
+struct LineWalk {
+  float e_ref, inv, slope, kv0;
+  int first, last;  // steps
+  float e;          // the next crossing, relative to the block's middle
+  float part[G];
+
+  __device__ __forceinline__ void load(const LineRay &r) {
+    e_ref = r.e_ref;
+    inv = r.inv;
+    slope = inv > 0.f ? __frcp_rn(inv) : 0.f;
+    kv0 = r.kv0;
+    first = (int)(r.rows & 0xffffu);
+    last = (int)(r.rows >> 16);
+  }
+  __device__ __forceinline__ bool empty() const { return first > last; }
+  __device__ __forceinline__ bool in_block(int blk) const { return first <= last && first >> 5 <= blk && blk <= last >> 5; }
+  // begins the block of steps from step0, in column c0 + the returned number
+  // (negative where the line has yet to reach c0)
+  __device__ __forceinline__ int enter(int step0, int n) {
+#pragma unroll
+    for (int m = 0; m < G; m++) part[m] = 0.f;
+    const float rel = e_ref - ((float)(step0 + 16) - 0.5f * (float)n);
+    float k = ceilf(fmaf(-16.f - rel, slope, -kv0));
+    e = fmaf(kv0 + k, inv, rel);
+    // the estimate is one off where a crossing nearly meets the block's start
+    const float d = e < -16.f ? 1.f : inv > 0.f && e - inv >= -16.f ? -1.f : 0.f;
+    k += d;
+    if (d != 0.f) e = fmaf(kv0 + k, inv, rel);
+    return (int)k;
+  }
+  // Step b of the block: the part of the row before the crossing, whether the
+  // ray crosses into the next column (and, if so, the crossing after that),
+  // and the sums, with a and c the pixels of the current and the next column.
+  // A crossing adds inv to e: within a block |e| stays below 17 (or is past the
+  // block), so the sums' rounding stays below that of e_ref.
+  __device__ __forceinline__ float before(float b) const { return __saturatef(e - (b - 16.f)); }
+  __device__ __forceinline__ bool crosses(float b) {
+    const bool x = e < b - 15.f;
+    if (x) e += inv;
+    return x;
+  }
+  __device__ __forceinline__ void add(float f, bool x, const typename Elem<G>::T &a, const typename Elem<G>::T &c) {
+    fma_elem<G>(part, f, a);
+    if (x) fma_elem<G>(part, 1.f - f, c);
+  }
+  __device__ __forceinline__ bool row(float b, const typename Elem<G>::T &a, const typename Elem<G>::T &c) {
+    const float f = before(b);
+    const bool x = crosses(b);
+    add(f, x, a, c);
+    return x;
+  }
+};
+
+// the Kahan total of a ray's block sums for one scan, and its line integral
+struct LineTotal {
+  float acc = 0.f, comp = 0.f;
+  __device__ __forceinline__ void fold(float part) { kahan_add(acc, comp, part); }
+  // with the ray's corrections: value(pixel) reads the scan's pixel x*n + y
+  template <typename V>
+  __device__ __forceinline__ float finish(const LineRay &r, const LineCorr *__restrict__ corr, V &&value) const {
+    float out = (acc - comp) * r.len;
+    const int nc = (int)(r.flags >> 8);
+    for (int k = 0; k < nc; k++) {
+      const LineCorr c = corr[r.corr0 + k];
+      out = fmaf(c.w, value(c.pix & ~kCorrForwardOnly), out);
+    }
+    return out;
+  }
+};
+
+// column c0, and the first element of a step's row in its copy
+__device__ __forceinline__ int line_c0(const LineRay &r, int n, int pitch) {
+  return r.off - ((r.flags & kLineSwap) ? n * pitch : 0) - kLinePad;
+}
+__device__ __forceinline__ int line_row_of(const LineRay &r, int step, int n) {
+  return (r.flags & kLineDown) ? n - 1 - step : step;
+}
+// no ray
+__device__ __forceinline__ LineRay line_none() {
+  LineRay r;
+  r.e_ref = r.inv = r.kv0 = r.len = 0.f;
+  r.off = r.corr0 = 0;
+  r.rows = 1u;
+  r.flags = 0u;
+  return r;
+}
+
+__device__ __forceinline__ LineRay load_line(const LineRay *p) {
+  const uint4 a = __ldg(reinterpret_cast<const uint4 *>(p)), b = __ldg(reinterpret_cast<const uint4 *>(p) + 1);
+  LineRay r;
+  r.e_ref = __uint_as_float(a.x);
+  r.inv = __uint_as_float(a.y);
+  r.kv0 = __uint_as_float(a.z);
+  r.len = __uint_as_float(a.w);
+  r.off = (int)b.x;
+  r.rows = b.y;
+  r.corr0 = (int)b.z;
+  r.flags = b.w;
+  return r;
+}
+
+}  // namespace medimg

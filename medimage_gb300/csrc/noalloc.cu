@@ -28,6 +28,8 @@
 namespace medimg {
 
 int fp_ctas(const ScanDev &S, int rpt);
+int fp_direct_ctas(const ScanDev &S, int threads);
+cudaError_t launch_fp_direct(const Launch &L, int threads, cudaStream_t st);
 cudaError_t launch_fp(const Launch &L, int kind, int rpt, int nctas, cudaStream_t st);
 
 namespace {
@@ -73,7 +75,11 @@ extern "C" __attribute__((visibility("default"))) int at_forward_residual_noallo
   std::memset(&L, 0, sizeof(L));
   fill_scan_plan(L.single, p);
   const int rpt = p.fp_rpt;  // the plan's autotuned forward-projector variant
-  const int nctas = fp_ctas(L.single, rpt);
+  // rays as lines: straight from the image; larger CTAs where the partial sums
+  // of small ones would not fit
+  const int max_ctas = (int)((kScratchBytes - kCtlBytes) / sizeof(double));
+  const int threads = !p.line_ok || fp_direct_ctas(L.single, 128) <= max_ctas ? 128 : 512;
+  const int nctas = p.line_ok ? fp_direct_ctas(L.single, threads) : fp_ctas(L.single, rpt);
   const size_t need = kCtlBytes + sizeof(double) * (size_t)nctas;
   if (need > kScratchBytes) {
     char msg[256];
@@ -101,7 +107,8 @@ extern "C" __attribute__((visibility("default"))) int at_forward_residual_noallo
   L.in_buf = B_F;
   L.out_buf = B_R;
   L.aux_buf = -1;
-  const cudaError_t e = launch_fp(L, p.kind, rpt, nctas, st);
+  const cudaError_t e =
+      p.line_ok ? launch_fp_direct(L, threads, st) : launch_fp(L, p.kind, rpt, nctas, st);
   if (e != cudaSuccess) return cuda_error(e, "no-alloc forward projection launch");
   AT_CUDA_TRY(cudaMemcpyAsync(d_energy, &ctl->e_data, sizeof(double), cudaMemcpyDeviceToDevice, st));
   return AT_OK;

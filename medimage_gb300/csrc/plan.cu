@@ -63,11 +63,32 @@ __device__ __forceinline__ void ray_endpoints(const RaySource &R, int view, int 
   dy = sdd * (dsin * scos + dcos * ssin) + sy;
 }
 
-// Traces ray (view, det).  Mode 0: fill the header and count segments.
-// Mode 1: also write the decision words into the block-interleaved array.
-template <int kMode, typename Real>
-__device__ void fan_trace_ray(const RaySource &R, int view, int det, RayHdr *hdr, int *offgrid, uint32_t *bits,
-                              uint32_t word_stride) {
+// The reference tracer's state where its segment loop begins
+// (tracing.cpp:39-115); empty: the ray misses the grid.
+template <typename Real>
+struct FanTrace {
+  Real sx, sy, ray_x, ray_y, L, len_x, len_y, lambda_min, lambda_max, lambda0, lambda_x, lambda_y;
+  int signx, signy, v_x, v_y;
+  bool empty;
+  // one step of the loop (tracing.cpp:118-146): crosses the nearer plane, x on ties
+  __device__ __forceinline__ bool step() {
+    const bool xstep = lambda_x <= lambda_y;
+    if (xstep) {
+      lambda0 = lambda_x;
+      lambda_x += len_x;
+      v_x += signx;
+    } else {
+      lambda0 = lambda_y;
+      lambda_y += len_y;
+      v_y += signy;
+    }
+    return xstep;
+  }
+};
+
+template <typename Real>
+__device__ FanTrace<Real> fan_trace_start(const RaySource &R, int view, int det) {
+  FanTrace<Real> T;
   const int NX = R.g.n, NY = R.g.n;
   const Real vx = (Real)R.g.pixel_mm, vy = (Real)R.g.pixel_mm;
   const Real zero = (Real)0.0, tiny = (Real)1.e-4, huge = (Real)1.e6;
@@ -99,23 +120,23 @@ __device__ void fan_trace_ray(const RaySource &R, int view, int det, RayHdr *hdr
   if (lambda_min == temp) index = 2;
   temp = (l0 > lN) ? l0 : lN;
   lambda_max = (lambda_max < temp) ? lambda_max : temp;
-
-  RayHdr h;
-  h.pix0 = 0;
-  h.nseg = 0;
-  h.xy0 = 0;
-  h.sgn = (signx > 0 ? 1 : 0) | (signy > 0 ? 2 : 0);
-  h.ax = h.ay = 0.f;
-  h.lenx = (float)len_x;
-  h.leny = (float)len_y;
-  if (lambda_min >= lambda_max) {
-    if (kMode == 0) {
-      *hdr = h;
-      *offgrid = 0;
-    }
-    return;
-  }
-  Real lambda0 = lambda_min, lambda_x, lambda_y;
+  T.sx = sx;
+  T.sy = sy;
+  T.ray_x = ray_x;
+  T.ray_y = ray_y;
+  T.L = L;
+  T.len_x = len_x;
+  T.len_y = len_y;
+  T.lambda_min = T.lambda0 = lambda_min;
+  T.lambda_max = lambda_max;
+  T.signx = signx;
+  T.signy = signy;
+  T.empty = lambda_min >= lambda_max;
+  T.lambda_x = T.lambda_y = zero;
+  T.v_x = T.v_y = 0;
+  if (T.empty) return T;
+  const Real lambda0 = lambda_min;
+  Real lambda_x, lambda_y;
   int v_x, v_y;
   if (index == 1) {  // tracing.cpp:91-102
     v_x = (signx == 1) ? 0 : NX - 1;
@@ -130,16 +151,45 @@ __device__ void fan_trace_ray(const RaySource &R, int view, int det, RayHdr *hdr
     tempx = (Real)v_x * vx;
     lambda_x = (absx < tiny) ? huge : (L * ((tempx + (Real)(signx > 0) * vx) - sx)) / (dx - sx);
   }
-  h.pix0 = v_x * NY + v_y;
-  h.xy0 = (v_x & 0xffff) | (v_y << 16);
-  h.ax = (float)(lambda_x - lambda_min);
-  h.ay = (float)(lambda_y - lambda_min);
+  T.lambda_x = lambda_x;
+  T.lambda_y = lambda_y;
+  T.v_x = v_x;
+  T.v_y = v_y;
+  return T;
+}
+
+// Traces ray (view, det).  Mode 0: fill the header and count segments.
+// Mode 1: also write the decision words into the block-interleaved array.
+template <int kMode, typename Real>
+__device__ void fan_trace_ray(const RaySource &R, int view, int det, RayHdr *hdr, int *offgrid, uint32_t *bits,
+                              uint32_t word_stride) {
+  const int NX = R.g.n, NY = R.g.n;
+  FanTrace<Real> T = fan_trace_start<Real>(R, view, det);
+  RayHdr h;
+  h.pix0 = 0;
+  h.nseg = 0;
+  h.xy0 = 0;
+  h.sgn = (T.signx > 0 ? 1 : 0) | (T.signy > 0 ? 2 : 0);
+  h.ax = h.ay = 0.f;
+  h.lenx = (float)T.len_x;
+  h.leny = (float)T.len_y;
+  if (T.empty) {
+    if (kMode == 0) {
+      *hdr = h;
+      *offgrid = 0;
+    }
+    return;
+  }
+  h.pix0 = T.v_x * NY + T.v_y;
+  h.xy0 = (T.v_x & 0xffff) | (T.v_y << 16);
+  h.ax = (float)(T.lambda_x - T.lambda_min);
+  h.ay = (float)(T.lambda_y - T.lambda_min);
   int numb = 0, bad = 0;
   uint32_t word = 0;
-  const Real stop = lambda_max - (Real)5.e-2;
-  while (lambda0 < stop) {  // tracing.cpp:118-146
-    if ((unsigned)v_x >= (unsigned)NX || (unsigned)v_y >= (unsigned)NY) bad++;
-    const bool xstep = lambda_x <= lambda_y;
+  const Real stop = T.lambda_max - (Real)5.e-2;
+  while (T.lambda0 < stop) {  // tracing.cpp:118-146
+    if ((unsigned)T.v_x >= (unsigned)NX || (unsigned)T.v_y >= (unsigned)NY) bad++;
+    const bool xstep = T.step();
     if (kMode == 1) {
       if (xstep) word |= 1u << (numb & 31);
       if ((numb & 31) == 31) {
@@ -148,21 +198,151 @@ __device__ void fan_trace_ray(const RaySource &R, int view, int det, RayHdr *hdr
       }
     }
     ++numb;
-    if (xstep) {
-      lambda0 = lambda_x;
-      lambda_x += len_x;
-      v_x += signx;
-    } else {
-      lambda0 = lambda_y;
-      lambda_y += len_y;
-      v_y += signy;
-    }
   }
   if (kMode == 1 && (numb & 31) != 0) bits[(size_t)(numb >> 5) * word_stride] = word;
   if (kMode == 0) {
     h.nseg = numb;
     *hdr = h;
     *offgrid = bad;
+  }
+}
+
+// Ray (view, det) as a line (LineRay, *out) with its corrections; returns how
+// many.  The traversal is walked again in FP64 and compared with the line: a
+// ray whose pixels do not all touch the line (to 1e-3 pixels), or whose length
+// in the grid is not the line's (an end point inside the grid, pixels off the
+// grid), gets no line and all its segments as corrections.  kFill 0 stores the
+// first correction in *corr, kFill 1 all of them.
+template <int kFill>
+__device__ int line_of_ray(const RaySource &R, int view, int det, int corr0, LineRay *out, LineCorr *corr) {
+  const int n = R.g.n;
+  const double px = R.g.pixel_mm;
+  LineRay o;
+  o.e_ref = 1e30f;
+  o.inv = o.kv0 = o.len = 0.f;
+  o.off = 0;
+  o.rows = 1u;  // first 1 > last 0
+  o.corr0 = corr0;
+  o.flags = 0u;
+  FanTrace<double> T = fan_trace_start<double>(R, view, det);
+  const double stop = T.lambda_max - 5.e-2;
+  if (T.empty || !(T.lambda0 < stop)) {
+    *out = o;
+    return 0;
+  }
+  const bool swap = fabs(T.ray_y) > fabs(T.ray_x);
+  const double su = (swap ? T.sy : T.sx) / px, sv = (swap ? T.sx : T.sy) / px;
+  const double slope = swap ? T.ray_x / T.ray_y : T.ray_y / T.ray_x;  // columns per row
+  const double len = px * sqrt(1.0 + slope * slope);
+  // stays in one column: the reference never crosses into the next where the
+  // ray's extent across is below 1e-4 (tracing.cpp:55-56)
+  const bool parallel = fabs(swap ? T.ray_x : T.ray_y) <= 1.e-4 || fabs(slope) * n < 1e-9;
+  const double inv = parallel ? 0.0 : 1.0 / slope;
+  const int v0 = swap ? T.v_x : T.v_y;
+  // rows of the crossings into the ray's first column from below and above,
+  // relative to the image's middle (the touch test, in FP32)
+  const float mid = 0.5f * n, finv = (float)inv;
+  const float flo = (float)(su + (v0 - sv) * inv) - mid, fhi = (float)(su + (v0 + 1 - sv) * inv) - mid;
+  bool regular = true;
+  int umin = n, umax = -1;
+  const double start = T.lambda0;
+  while (T.lambda0 < stop) {
+    const int u = swap ? T.v_y : T.v_x, v = swap ? T.v_x : T.v_y;
+    T.step();
+    const float dv = (float)(v - v0), uc = (float)u - mid;
+    const float ea = fmaf(dv, finv, flo) - uc, eb = fmaf(dv, finv, fhi) - uc;
+    // a shallow ray's crossings are known to 1e-3 columns, i.e. 1e-3 inv rows
+    const float tol = 1e-3f + 1e-3f * fabsf(finv);
+    const bool touch = parallel ? v == v0 : fminf(ea, eb) <= 1.f + tol && fmaxf(ea, eb) >= -tol;
+    regular &= (unsigned)u < (unsigned)n && (unsigned)v < (unsigned)n && touch;
+    umin = min(umin, u);
+    umax = max(umax, u);
+  }
+  // the rest of the line in the grid: what the reference leaves out
+  const FanTrace<double> Tend = T;
+  int nc = 0;
+  while ((unsigned)T.v_x < (unsigned)n && (unsigned)T.v_y < (unsigned)n && nc <= 64) {
+    const int u = swap ? T.v_y : T.v_x;
+    umin = min(umin, u);
+    umax = max(umax, u);
+    T.step();
+    nc++;
+  }
+  double lo = 0.0, hi = n;
+  if (!parallel) {
+    const double a = su + (0 - sv) * inv, b = su + (n - sv) * inv;
+    lo = fmax(lo, fmin(a, b));
+    hi = fmin(hi, fmax(a, b));
+  }
+  regular = regular && nc <= 64 && fabs((hi - lo) * len - (T.lambda0 - start)) < 1e-5 * px;
+  if (!regular) {
+    int k = 0;
+    T = fan_trace_start<double>(R, view, det);
+    while (T.lambda0 < stop) {
+      const int64_t flat = (int64_t)T.v_x * n + T.v_y;
+      const bool in = (unsigned)T.v_x < (unsigned)n && (unsigned)T.v_y < (unsigned)n;
+      const double l0 = T.lambda0;
+      T.step();
+      // the reference reads any linear index inside the image (its
+      // get_img_addr), and back projects what is on the grid
+      if (flat < 0 || flat >= (int64_t)n * n) continue;
+      if (kFill || k == 0) corr[k] = LineCorr{(int32_t)flat | (in ? 0 : kCorrForwardOnly), (float)(T.lambda0 - l0)};
+      k++;
+    }
+    o.flags = (uint32_t)k << 8;
+    *out = o;
+    return k;
+  }
+  T = Tend;
+  for (int k = 0; k < nc; k++) {
+    const int flat = T.v_x * n + T.v_y;
+    const double l0 = T.lambda0;
+    T.step();
+    if (kFill || k == 0) corr[k] = LineCorr{flat, (float)(l0 - T.lambda0)};
+  }
+  // walked so that the columns increase
+  const bool down = slope < 0.0;
+  int c0 = v0;
+  if (!parallel) {
+    const double vs = sv + ((down ? umax + 1 : umin) - su) * slope, ve = sv + ((down ? umin : umax + 1) - su) * slope;
+    c0 = max(-1, min(n, (int)floor(vs)));
+    const int ce = max(-1, min(n, (int)ceil(ve) - 1));
+    const int half = max(0, ce - c0) / 2;
+    const double e = su + (c0 + 1 + half - sv) * inv - 0.5 * n;
+    o.e_ref = (float)(down ? -e : e);
+    o.inv = (float)fabs(inv);
+    o.kv0 = (float)-half;
+  }
+  // one row more at either end, where the walk's rounding may still find a
+  // sliver of the ray
+  const int first = down ? n - 1 - umax : umin, last = down ? n - 1 - umin : umax;
+  o.len = (float)len;
+  o.off = (swap ? n * line_pitch(n) : 0) + c0 + kLinePad;
+  o.rows = (uint32_t)max(first - 1, 0) | ((uint32_t)min(last + 1, n - 1) << 16);
+  o.flags = (swap ? kLineSwap : 0u) | (down ? kLineDown : 0u) | ((uint32_t)nc << 8);
+  *out = o;
+  return nc;
+}
+
+// every ray's line, its first correction and how many it has
+__global__ void line_rays_kernel(const RaySource R, LineRay *line, LineCorr *first, int *count) {
+  const int ray = blockIdx.x * blockDim.x + threadIdx.x;
+  if (ray >= R.g.nviews * R.g.ndets) return;
+  count[ray] = line_of_ray<0>(R, ray / R.g.ndets, ray % R.g.ndets, 0, line + ray, first + ray);
+}
+
+// the corrections in ray order; rays with several are traced once more
+__global__ void line_corr_kernel(const RaySource R, const LineCorr *first, const int *off, LineRay *line,
+                                 LineCorr *corr) {
+  const int ray = blockIdx.x * blockDim.x + threadIdx.x;
+  if (ray >= R.g.nviews * R.g.ndets) return;
+  const int o = off[ray], c = off[ray + 1] - o;
+  if (c == 0) return;
+  if (c == 1) {
+    line[ray].corr0 = o;
+    corr[o] = first[ray];
+  } else {
+    line_of_ray<1>(R, ray / R.g.ndets, ray % R.g.ndets, o, line + ray, corr + o);
   }
 }
 
@@ -402,6 +582,51 @@ int build_fan_runs(Plan &p, cudaStream_t st) {
   return AT_OK;
 }
 
+// The rays as lines; none for the plain FP32 traversal (its pixels are those
+// of its own arithmetic) and where corrections would outweigh the lines.
+int build_lines(Plan &p, const RaySource &R, cudaStream_t st) {
+  if (p.alpha_fp32) return AT_OK;
+  const int nrays = p.nviews * p.ndets, tpb = 128;
+  int *cnt_d = nullptr;
+  LineCorr *first = nullptr;
+  LineRay *line = nullptr;
+  const auto free_temps = scope_exit([&] {
+    cudaFree(cnt_d);
+    cudaFree(first);
+    cudaFree(line);
+  });
+  AT_CUDA_TRY(cudaMalloc(&cnt_d, sizeof(int) * ((size_t)nrays + 1)));
+  AT_CUDA_TRY(cudaMalloc(&first, sizeof(LineCorr) * (size_t)nrays));
+  AT_CUDA_TRY(cudaMalloc(&line, sizeof(LineRay) * (size_t)nrays));
+  line_rays_kernel<<<(nrays + tpb - 1) / tpb, tpb, 0, st>>>(R, line, first, cnt_d);
+  AT_CUDA_TRY(cudaGetLastError());
+  std::vector<int> off((size_t)nrays + 1);
+  AT_CUDA_TRY(cudaMemcpyAsync(off.data(), cnt_d, sizeof(int) * nrays, cudaMemcpyDeviceToHost, st));
+  AT_CUDA_TRY(cudaStreamSynchronize(st));
+  int64_t tot = 0;
+  for (int r = 0; r < nrays; r++) {
+    const int c = off[r];
+    off[r] = (int)tot;
+    tot += c;
+    // a ray leaves out one piece at most where pixels are wider than 0.05 mm;
+    // the rest are whole rays, a pixel at a time
+    if (tot > nrays + p.segments / 16 || tot >= (1ll << 30)) return AT_OK;
+  }
+  off[nrays] = (int)tot;
+  int rc;
+  if ((rc = dev_alloc(&p.lcorr_d, tot, p.device_bytes))) return rc;
+  AT_CUDA_TRY(cudaMemcpyAsync(cnt_d, off.data(), sizeof(int) * ((size_t)nrays + 1), cudaMemcpyHostToDevice, st));
+  line_corr_kernel<<<(nrays + tpb - 1) / tpb, tpb, 0, st>>>(R, first, cnt_d, line, p.lcorr_d);
+  AT_CUDA_TRY(cudaGetLastError());
+  AT_CUDA_TRY(cudaStreamSynchronize(st));
+  p.line_d = line;
+  line = nullptr;
+  p.device_bytes += (int64_t)sizeof(LineRay) * nrays;
+  p.ncorr = tot;
+  p.line_ok = 1;
+  return AT_OK;
+}
+
 int build_fan_plan(Plan &p, cudaStream_t st, const double *h_ends) {
   const at_fan_geometry &g = p.geom;
   const int nv = g.nviews, nd = g.ndets, nrays = nv * nd;
@@ -492,6 +717,7 @@ int build_fan_plan(Plan &p, cudaStream_t st, const double *h_ends) {
     fan_fill_kernel<double><<<(nrays + tpb - 1) / tpb, tpb, 0, st>>>(R, p.nblocks_per_view, p.blk_word_d, p.bits_d);
   AT_CUDA_TRY(cudaGetLastError());
 
+  if ((rc = build_lines(p, R, st))) return rc;
   if ((rc = build_fan_runs(p, st))) return rc;
   AT_CUDA_TRY(cudaStreamSynchronize(st));
   cudaFree(tab_d);
@@ -723,6 +949,8 @@ Plan::~Plan() {
   cudaFree(bits_d);
   cudaFree(blk_word_d);
   cudaFree(blk_off_d);
+  cudaFree(line_d);
+  cudaFree(lcorr_d);
   cudaFree(run_d);
   cudaFree(tile_off_d);
   cudaFree(gc_seg_d);

@@ -1,7 +1,9 @@
 // project.cu -- forward (A f) and back (A^T r) projection kernels with the
 // solver's fused epilogues.
 //
-// Fan beam, forward: each thread walks RPT adjacent rays of one view through
+// Fan beam, forward: each thread walks a ray row by row along its line (LineRay,
+// line.cuh).  Plans without lines (the plain FP32 traversal, ray tables that
+// are mostly no lines): each thread walks RPT adjacent rays of one view through
 // the plan's decision bits (1 bit per segment, block-interleaved so a warp's
 // word loads are coalesced), reads the traversed pixels through the read-only
 // cache, accumulates FP32 products per 32-segment word and folds the word sums
@@ -20,8 +22,10 @@
 
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 
 #include "epilogue.cuh"
+#include "line.cuh"
 #include "solver.h"
 
 namespace medimg {
@@ -57,30 +61,43 @@ __device__ __forceinline__ T pack_elem(const float *const (&src)[kGroupMax], int
   else return make_float4(v[0], v[1], v[2], v[3]);
 }
 
+// The zeros beside the columns of the padded copies (ScanDev::lpad): rows
+// r0..r0+31 of the copy at pk, by 256 threads
+template <typename T>
+__device__ __forceinline__ void pack_guards(T *pk, int n, int pitch, int pad, int r0) {
+  const int g = pitch - n;
+  for (int i = threadIdx.y * blockDim.x + threadIdx.x; i < 32 * g; i += 256) {
+    const int r = r0 + i / g, k = i % g;
+    if (r < n) pk[(size_t)r * pitch + (k < pad ? k : n + k)] = T{};
+  }
+}
+
 // Images of a scan (or a group) into its pack buffer, row-major and transposed,
 // 32 x 32 pixels at a time through shared memory so that both copies are
 // written in whole rows: tiles (local, local + ncta, ...) of the scan's CTAs.
 template <typename T>
-__device__ __forceinline__ void pack_image_tiles(const float *const (&src)[kGroupMax], int n, T *pk, int local,
-                                                 int ncta, float4 (*raw)[33]) {
+__device__ __forceinline__ void pack_image_tiles(const float *const (&src)[kGroupMax], int n, int pitch, int pad,
+                                                 T *pk, int local, int ncta, float4 (*raw)[33]) {
   T(*tile)[33] = reinterpret_cast<T(*)[33]>(raw);  // 32 x 33 elements of T
   const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;  // 8 rows of 32 threads
   const int tiles_y = (n + 31) / 32;
-  const size_t npix = (size_t)n * n;
+  T *pkt = pk + (size_t)n * pitch;
   for (int t = local; t < tiles_y * tiles_y; t += ncta) {
     const int x0 = (t / tiles_y) * 32, y0 = (t % tiles_y) * 32;
     for (int r = row; r < 32; r += 8) {
       const int x = x0 + r, y = y0 + lane;
       if (x < n && y < n) {
         const T v = pack_elem<T>(src, x * n + y);
-        pk[(size_t)x * n + y] = v;
+        pk[(size_t)x * pitch + pad + y] = v;
         tile[r][lane] = v;
       }
     }
+    if (pad && y0 == 0) pack_guards(pk, n, pitch, pad, x0);
+    if (pad && x0 == 0) pack_guards(pkt, n, pitch, pad, y0);
     __syncthreads();
     for (int r = row; r < 32; r += 8) {
       const int y = y0 + r, x = x0 + lane;
-      if (x < n && y < n) pk[npix + (size_t)y * n + x] = tile[lane][r];
+      if (x < n && y < n) pkt[(size_t)y * pitch + pad + x] = tile[lane][r];
     }
     __syncthreads();
   }
@@ -111,9 +128,12 @@ __global__ void __launch_bounds__(256) fp_pack_kernel(const Launch L, int bins) 
   const int local = blockIdx.x - cta0;
   if (!bins) {
     __shared__ float4 raw[32][33];
-    if (S.nmem == 1) pack_image_tiles<float>(src, S.n, reinterpret_cast<float *>(S.pack), local, ncta, raw);
-    else if (S.nmem == 2) pack_image_tiles<float2>(src, S.n, reinterpret_cast<float2 *>(S.pack), local, ncta, raw);
-    else pack_image_tiles<float4>(src, S.n, S.pack, local, ncta, raw);
+    if (S.nmem == 1)
+      pack_image_tiles<float>(src, S.n, S.lpitch, S.lpad, reinterpret_cast<float *>(S.pack), local, ncta, raw);
+    else if (S.nmem == 2)
+      pack_image_tiles<float2>(src, S.n, S.lpitch, S.lpad, reinterpret_cast<float2 *>(S.pack), local, ncta, raw);
+    else
+      pack_image_tiles<float4>(src, S.n, S.lpitch, S.lpad, S.pack, local, ncta, raw);
     return;
   }
   for (int p = local * blockDim.x + threadIdx.x; p < S.nbins; p += ncta * blockDim.x) {
@@ -130,6 +150,7 @@ template <int RPT, int G>
 __device__ __forceinline__ void fan_fp_body(const Launch &L, const int unit) {
   const int scan = L.scans ? find_scan(L.prefix, L.nscans, unit) : 0;
   const ScanDev &S = scan_of(L, scan);
+  if (S.line) return;  // line_fp_body's
   const int nm = L.scans ? S.nmem : 1;
   const ScanDev *M[G];
   bool act[G];
@@ -383,6 +404,175 @@ __global__ void __launch_bounds__(128, 7) fan_fp_kernel<1, 4>(const Launch L) {
 template <int RPT, int G>
 __global__ void __launch_bounds__(128) fan_fp_queue_kernel(const Launch L) {
   persistent_loop(L, [&](int unit) { fan_fp_body<RPT, G>(L, unit); });
+}
+
+
+// The same projection from the rays' lines (LineRay): a thread steps its ray
+// row by row along the axis it runs closer to.  All lanes of a warp are in the
+// same row of the same copy at any time, so their 16 + 16 pixels (the warp's
+// two views) lie side by side in one row: about two cache lines, where the
+// lanes of the segment walk, at equal step counts but in a dozen different
+// rows, touch about ten.  A row costs two gathers (current and next column; a
+// predicated second one measured slower) and no decision bits.
+// Bound: instruction issue and load latency for one member (58 % issue, 44 %
+// L1 at C2), the L1 data path for four (84 %: 2 x 16 bytes a row and lane).
+// C2, the image's copies included: one slice 243 -> 130 us, eight slices
+// 812 -> 560 us; error against 64 bits 2.2e-7 -> 1.3e-7.
+// kDirect: the image itself instead of the padded copies, every column checked
+// (the call that may not allocate); the same sums.
+template <int G, bool kDirect>
+__device__ __forceinline__ void line_fp_body(const Launch &L, const int unit) {
+  using T = typename Elem<G>::T;
+  static_assert(G == 1 || !kDirect, "groups read their interleaved copies");
+  const int scan = L.scans ? find_scan(L.prefix, L.nscans, unit) : 0;
+  const ScanDev &S = scan_of(L, scan);
+  if (!S.line) return;  // fan_fp_body's
+  // the group's members and which of them this launch serves (read again for
+  // the epilogue, so that they hold no registers through the walk)
+  auto members = [&](const ScanDev *(&M)[G], bool(&act)[G]) {
+    const int nm = L.scans ? S.nmem : 1;
+    bool any = false;
+#pragma unroll
+    for (int m = 0; m < G; m++) {
+      M[m] = L.scans ? &L.scans[S.mem[m < nm ? m : 0]] : &L.single;
+      act[m] = m < nm && flow_active(*M[m], L.flow);
+      any |= act[m];
+    }
+    return any;
+  };
+  {
+    const ScanDev *M[G];
+    bool act[G];
+    if (!members(M, act)) return;
+  }
+  const int cta0 = L.scans ? __ldg(L.prefix + scan) : 0;
+  const int local_cta = unit - cta0;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int n = S.n, pitch = S.lpitch;
+  // 16 adjacent rays of each of two neighbouring views per warp, four and four
+  // of them per quarter warp (a 16-byte gather goes out by quarter warps: C2,
+  // eight slices 529 us against 567 with eight rays of one view).  Four warps
+  // take 32 detectors of two neighbouring view pairs, whose rays nearly
+  // coincide.  All views of the middle detectors first, whose rays are the
+  // longest, then outwards: short rays end the launch (C2: 207 -> 128 us
+  // together with the unconditional second gather).
+  const int lw = local_cta * (int)(blockDim.x >> 5) + warp;
+  const int nq = (S.nviews + 3) >> 2, ng = S.nbpv * 4;
+  const int g = (lw >> 2) / nq, vq = (lw >> 2) - g * nq;
+  const int view = g < ng ? 4 * vq + 2 * (lw & 1) + ((lane >> 2) & 1) : S.nviews;
+  const int det = (ng / 2 + ((g & 1) ? -((g + 1) >> 1) : g >> 1)) * 32 + (lw & 2) * 8 + (lane >> 3) * 4 + (lane & 3);
+  const bool valid = view < S.nviews && det < S.ndets;
+  const float *__restrict__ img = S.buf[L.in_buf];
+  const T *__restrict__ pk = reinterpret_cast<const T *>(S.pack);
+  const LineRay ray = valid ? load_line(S.line + (size_t)view * S.ndets + det) : line_none();
+  LineWalk<G> w;
+  w.load(ray);
+  const bool swap = (ray.flags & kLineSwap) != 0, down = (ray.flags & kLineDown) != 0, none = w.empty();
+  // The lane's copy and its rows in walk order: element row0 + step * stride +
+  // (padded) column.  A lane without a line reads the zeros at element 0.
+  const int c0 = none ? -kLinePad : line_c0(ray, n, line_pitch(n));
+  const int row0 = none ? 0 : (swap ? n * pitch : 0) + (down ? (n - 1) * pitch : 0);
+  const int stride = none ? 0 : down ? -pitch : pitch;
+  // kDirect: rows and columns of the image itself
+  const int drow0 = down ? (n - 1) * (swap ? 1 : n) : 0, dstride = (swap ? 1 : n) * (down ? -1 : 1), dcol = swap ? n : 1;
+  auto direct = [&](int step, int c) { return (unsigned)c < (unsigned)n ? __ldg(img + drow0 + step * dstride + c * dcol) : 0.f; };
+  // blocks, from the first any lane has to the last
+  const int blk0 = (int)__reduce_min_sync(0xffffffffu, none ? 0xffffu : (unsigned)w.first >> 5);
+  const int blk1 = (int)__reduce_max_sync(0xffffffffu, none ? 0u : (unsigned)(w.last >> 5) + 1u);
+  // Rows are taken kBatch at a time: the crossings and the pixels first (the
+  // crossings need none), then the sums.  One to four rows measure within 3 %
+  // of each other.
+  constexpr int kBatch = G;
+  auto walk_block = [&](int step0) {
+    int c = c0 + w.enter(step0, n);
+    if constexpr (kDirect) {
+      for (int b = 0; b < min(32, n - step0); b++)
+        c += w.row((float)b, direct(step0 + b, c), direct(step0 + b, c + 1)) ? 1 : 0;
+    } else {
+      int off = row0 + step0 * stride;  // the step's row
+      const bool in = none || (w.first <= step0 && step0 + 31 <= w.last);
+      // a column's place in its row; any off the grid (as a line is before and
+      // behind its rows) reads the zeros beside the last one
+      auto any_column = [&](int col) { return (int)min((unsigned)(col + kLinePad), (unsigned)(n + kLinePad + 1)); };
+      // rows b..b+kBatch-1: inside, off is the pixel; else the row
+      auto rows = [&](int b, auto inside) {
+        float f[kBatch];
+        bool x[kBatch];
+        T va[kBatch], vc[kBatch];
+#pragma unroll
+        for (int i = 0; i < kBatch; i++) {
+          f[i] = w.before((float)(b + i));
+          const int at = inside ? off : off + any_column(c);
+          va[i] = __ldg(pk + at);
+          vc[i] = __ldg(pk + at + 1);
+          x[i] = w.crosses((float)(b + i));
+          if (inside) off += x[i] ? 1 : 0;
+          else c += x[i] ? 1 : 0;
+          off += stride;
+        }
+#pragma unroll
+        for (int i = 0; i < kBatch; i++)
+          w.add(f[i], x[i], va[i], vc[i]);
+      };
+      if (__all_sync(0xffffffffu, in)) {
+        off += c + kLinePad;
+#pragma unroll
+        for (int b = 0; b < 32; b += kBatch) rows(b, std::true_type{});
+      } else if (step0 + 32 <= n) {
+#pragma unroll
+        for (int b = 0; b < 32; b += kBatch) rows(b, std::false_type{});
+      } else {
+        for (int b = 0; b < n - step0; b++) {
+          const int at = off + any_column(c);
+          c += w.row((float)b, __ldg(pk + at), __ldg(pk + at + 1)) ? 1 : 0;
+          off += stride;
+        }
+      }
+    }
+  };
+  LineTotal tot[G];
+  for (int blk = blk0; blk < blk1; blk++) {
+    walk_block(blk << 5);
+    if (w.in_block(blk))
+#pragma unroll
+      for (int m = 0; m < G; m++) tot[m].fold(w.part[m]);
+  }
+  const ScanDev *M[G];
+  bool act[G];
+  members(M, act);
+  const int ncta = L.scans ? __ldg(L.prefix + scan + 1) - cta0 : gridDim.x;
+  const LineRay end = valid ? load_line(S.line + (size_t)view * S.ndets + det) : line_none();
+  FF s0[G];
+#pragma unroll
+  for (int m = 0; m < G; m++) {
+    s0[m] = ff_zero();
+    if (!valid || !act[m]) continue;
+    const float out = tot[m].finish(end, S.lcorr, [&](int p) {
+      if constexpr (kDirect) return __ldg(img + p);
+      else return __ldg(reinterpret_cast<const float *>(pk + (p / n) * pitch + kLinePad + p % n) + m);
+    });
+    fp_epilogue(*M[m], L, view * S.ndets + det, out, s0[m]);
+  }
+  if (stage_reduces(L.stage)) {
+    if constexpr (G == 1) {
+      reduce_and_finalize<1>(*M[0], L, s0, local_cta, ncta);
+    } else {
+      unsigned mask = 0;
+#pragma unroll
+      for (int m = 0; m < G; m++) mask |= act[m] ? 1u << m : 0u;
+      reduce_and_finalize_group<G>(M, mask, L, s0, local_cta, ncta);
+    }
+  }
+}
+
+template <int G>
+__global__ void __launch_bounds__(128) line_fp_kernel(const Launch L) {
+  line_fp_body<G, false>(L, blockIdx.x);
+}
+__global__ void __launch_bounds__(512) line_fp_direct_kernel(const Launch L) { line_fp_body<1, true>(L, blockIdx.x); }
+template <int G>
+__global__ void __launch_bounds__(128) line_fp_queue_kernel(const Launch L) {
+  persistent_loop(L, [&](int unit) { line_fp_body<G, false>(L, unit); });
 }
 
 
@@ -966,9 +1156,9 @@ __global__ void __launch_bounds__(256) gc_bp_kernel(const Launch L) {
 // ---------------------------------------------------------------------------
 int cone_ctas(const ScanDev &S);
 cudaError_t launch_cone_fp(const Launch &L, int nctas, cudaStream_t st);
-cudaError_t launch_fp_slab(const Launch &L, int G, int nctas, int threads, size_t smem, cudaStream_t st);
+int launch_fp_slab(const Launch &L, int G, int nctas, int threads, size_t smem, cudaStream_t st);
 size_t slab_smem_bytes(int G, int rows, int wbox);
-int encode_pack_tmap(CUtensorMap *out, const void *pack, int n, int G, int wbox, int rows);
+int encode_pack_tmap(CUtensorMap *out, const void *pack, int n, int pitch, int G, int wbox, int rows);
 cudaError_t launch_cone_bp(const Launch &L, int nctas, const Launch &Lpix, int pix_nctas, cudaStream_t st);
 
 // CTAs of `kernel` (with `threads` threads) resident on the whole device at
@@ -996,9 +1186,16 @@ void launch_maybe_queued(K kernel, K qkernel, int &resident, const Launch &L, in
   }
 }
 
+// CTAs of a forward projection along lines, with `threads` threads each
+int line_ctas(const ScanDev &S, int threads) {
+  const int w = threads / 32;
+  return ((S.nviews + 3) / 4 * 4 * S.nbpv * 4 + w - 1) / w;
+}
+
 int fp_ctas(const ScanDev &S, int rpt) {
   if (S.kind == AT_GEOM_GOLDNC) return (kGcFpWarps + 3) / 4;
   if (S.kind == AT_GEOM_CONE) return cone_ctas(S);
+  if (S.line) return line_ctas(S, 128);
   // one ray per thread: warps of two views (an odd view count adds a half-empty pair)
   const int views = rpt == 1 ? (S.nviews + 1) / 2 * 2 : S.nviews;
   const int warps = views * S.nbpv * (4 / rpt);
@@ -1008,6 +1205,7 @@ int fp_ctas(const ScanDev &S, int rpt) {
 // CTAs of a grouped forward projection (one ray per thread)
 int fp_group_ctas(const ScanDev &S) {
   if (S.kind != AT_GEOM_FAN && S.kind != AT_GEOM_RAYS) return 0;
+  if (S.line) return line_ctas(S, kFpGroupThreads);
   constexpr int w = kFpGroupThreads / 32;
   static_assert(kFpGroupThreads == 128, "a grouped CTA holds four warps (two views x 64 rays)");
   return ((S.nviews + 1) / 2 * 2 * S.nbpv * 4 + w - 1) / w;
@@ -1032,12 +1230,23 @@ int bp_split_for(int tiles, int nvb) {
 
 int pix_ctas(const ScanDev &S) { return ((S.n + kPixRows - 1) / kPixRows) * ((S.n + 31) / 32) * S.nz; }
 
-cudaError_t launch_fp(const Launch &L, int kind, int rpt, int nctas, cudaStream_t st) {
-  if (kind == AT_GEOM_GOLDNC) {
-    gc_fp_kernel<<<nctas, 128, 0, st>>>(L);
-  } else if (kind == AT_GEOM_CONE) {
-    return launch_cone_fp(L, nctas, st);
-  } else if (rpt == 4) {
+// the forms of a launch's scans (Launch::forms)
+int line_ctas(const ScanDev &S, int threads);
+
+int launch_forms(const Launch &L) { return L.scans ? L.forms : L.single.line ? 2 : 1; }
+
+// Fan-beam / ray-table scans: the walk along lines (the scans' pack buffers
+// hold padded copies) for scans with lines, the walk by decision bits for the
+// others; in a batch with both, each kernel's CTAs of the other's scans return
+// at once.  Returns the launches.
+int launch_fp_walk(const Launch &L, int rpt, int nctas, cudaStream_t st) {
+  const int forms = launch_forms(L);
+  if (forms & 2) {
+    static int res = 0;
+    launch_maybe_queued(line_fp_kernel<1>, line_fp_queue_kernel<1>, res, L, nctas, 128, st);
+  }
+  if (!(forms & 1)) return 1;
+  if (rpt == 4) {
     static int res = 0;
     launch_maybe_queued(fan_fp_kernel<4, 1>, fan_fp_queue_kernel<4, 1>, res, L, nctas, 128, st);
   } else if (rpt == 2) {
@@ -1047,9 +1256,27 @@ cudaError_t launch_fp(const Launch &L, int kind, int rpt, int nctas, cudaStream_
     static int res = 0;
     launch_maybe_queued(fan_fp_kernel<1, 1>, fan_fp_queue_kernel<1, 1>, res, L, nctas, 128, st);
   }
+  return forms == 3 ? 2 : 1;
+}
+
+// CTAs of a forward projection without copies of the image, with `threads` threads each
+int fp_direct_ctas(const ScanDev &S, int threads) { return line_ctas(S, threads); }
+
+cudaError_t launch_fp_direct(const Launch &L, int threads, cudaStream_t st) {
+  line_fp_direct_kernel<<<fp_direct_ctas(L.single, threads), threads, 0, st>>>(L);
   return cudaGetLastError();
 }
 
+cudaError_t launch_fp(const Launch &L, int kind, int rpt, int nctas, cudaStream_t st) {
+  if (kind == AT_GEOM_GOLDNC) {
+    gc_fp_kernel<<<nctas, 128, 0, st>>>(L);
+  } else if (kind == AT_GEOM_CONE) {
+    return launch_cone_fp(L, nctas, st);
+  } else {
+    launch_fp_walk(L, rpt, nctas, st);
+  }
+  return cudaGetLastError();
+}
 // Forward projection of a batch whose scans sharing a plan are grouped: the
 // members' inputs are interleaved (over the pixel-pass CTAs of Lpix), then
 // each group's rays are walked once, one ray per thread, in one launch per
@@ -1065,62 +1292,75 @@ int launch_fp_group(const Launch &L, const Launch &Lpix, const Launch &L1, const
     const int nc[3] = {nctas, nctas1, nctas2};
     for (int i = 0; i < 3; i++) {
       if (nc[i] <= 0) continue;
-      const cudaError_t e = launch_fp_slab(*Ls[i], G[i], nc[i], slab->threads, slab->smem[i], st);
-      if (e != cudaSuccess) return -1;
-      n++;
+      const int nl = launch_fp_slab(*Ls[i], G[i], nc[i], slab->threads, slab->smem[i], st);
+      if (nl < 0) return -1;
+      n += nl;
     }
     return n;
   }
   Launch Lg = L, Lg1 = L1, Lg2 = L2;
   Lg.tr = Lg1.tr = Lg2.tr = 1;
-  static int res4 = 0, res1 = 0, res2 = 0;
-  launch_maybe_queued(fan_fp_kernel<1, kGroupMax>, fan_fp_queue_kernel<1, kGroupMax>, res4, Lg, nctas,
-                      kFpGroupThreads, st);
-  launch_maybe_queued(fan_fp_kernel<1, 1>, fan_fp_queue_kernel<1, 1>, res1, Lg1, nctas1, kFpGroupThreads, st);
-  launch_maybe_queued(fan_fp_kernel<1, 2>, fan_fp_queue_kernel<1, 2>, res2, Lg2, nctas2, kFpGroupThreads, st);
-  return n + (nctas > 0) + (nctas1 > 0) + (nctas2 > 0);
+  if (L.forms & 2) {
+    static int res4 = 0, res1 = 0, res2 = 0;
+    launch_maybe_queued(line_fp_kernel<kGroupMax>, line_fp_queue_kernel<kGroupMax>, res4, Lg, nctas, kFpGroupThreads,
+                        st);
+    launch_maybe_queued(line_fp_kernel<1>, line_fp_queue_kernel<1>, res1, Lg1, nctas1, kFpGroupThreads, st);
+    launch_maybe_queued(line_fp_kernel<2>, line_fp_queue_kernel<2>, res2, Lg2, nctas2, kFpGroupThreads, st);
+  }
+  if (L.forms & 1) {
+    static int res4 = 0, res1 = 0, res2 = 0;
+    launch_maybe_queued(fan_fp_kernel<1, kGroupMax>, fan_fp_queue_kernel<1, kGroupMax>, res4, Lg, nctas,
+                        kFpGroupThreads, st);
+    launch_maybe_queued(fan_fp_kernel<1, 1>, fan_fp_queue_kernel<1, 1>, res1, Lg1, nctas1, kFpGroupThreads, st);
+    launch_maybe_queued(fan_fp_kernel<1, 2>, fan_fp_queue_kernel<1, 2>, res2, Lg2, nctas2, kFpGroupThreads, st);
+  }
+  return n + ((nctas > 0) + (nctas1 > 0) + (nctas2 > 0)) * (L.forms == 3 ? 2 : 1);
 }
 
-// out[p] = in[p] and out[n*n + y*n + x] = in[x*n + y] for an n x n image
-// (the row-major and transposed copies the forward projectors read), through
-// 32 x 32 shared-memory tiles (coalesced reads and writes)
+// The row-major and transposed copies of an n x n image that the forward
+// projectors read (lpitch and lpad as in ScanDev), through 32 x 32 shared-memory
+// tiles (coalesced reads and writes)
 __global__ void __launch_bounds__(256) pack_single_kernel(const float *__restrict__ in, float *__restrict__ out,
-                                                           int n) {
+                                                           int n, int pitch, int pad) {
   __shared__ float t[32][33];
   const int bx = blockIdx.x * 32, by = blockIdx.y * 32;
-  const size_t npix = (size_t)n * n;
+  float *outt = out + (size_t)n * pitch;
   for (int r = threadIdx.y; r < 32; r += 8) {
     const int x = by + r, y = bx + threadIdx.x;
     if (x < n && y < n) {
       const float v = in[(size_t)x * n + y];
       t[r][threadIdx.x] = v;
-      out[(size_t)x * n + y] = v;
+      out[(size_t)x * pitch + pad + y] = v;
     }
   }
+  if (pad && bx == 0) pack_guards(out, n, pitch, pad, by);
+  if (pad && by == 0) pack_guards(outt, n, pitch, pad, bx);
   __syncthreads();
   for (int r = threadIdx.y; r < 32; r += 8) {
     const int y = bx + r, x = by + threadIdx.x;
-    if (x < n && y < n) out[npix + (size_t)y * n + x] = t[threadIdx.x][r];
+    if (x < n && y < n) outt[(size_t)y * pitch + pad + x] = t[threadIdx.x][r];
   }
 }
 
 // Device scratch of one fan-beam / ray-table forward projection outside a
-// batch: the image's two copies (2 n^2 floats) and, for the slab projector,
-// its TMA descriptor.
+// batch: the image's two copies and, for the slab projector, its TMA
+// descriptor.
 size_t fp_single_scratch_bytes(const Plan &p) {
-  return ((sizeof(float) * 2 * (size_t)p.n * p.n + 255) & ~(size_t)255) + sizeof(CUtensorMap);
+  const size_t pitch = p.line_ok ? line_pitch(p.n) : p.n;
+  return ((sizeof(float) * 2 * (size_t)p.n * pitch + 255) & ~(size_t)255) + sizeof(CUtensorMap);
 }
 
 // One fan-beam / ray-table forward projection outside a batch: the image's
 // row-major and transposed copies into `scratch` (fp_single_scratch_bytes),
-// then the slab projector when the plan has slab tables, else the L1 walk
-// reading the transposed copy where rays run closer to the y axis.  The TMA
-// descriptor is copied from host memory that lives only through this call:
-// pageable cudaMemcpyAsync stages it before returning.
+// then the slab projector when the plan has slab tables, else the L1 walk.
+// The TMA descriptor is copied from host memory that lives only through this
+// call: pageable cudaMemcpyAsync stages it before returning.
 cudaError_t launch_fp_single(const Launch &L, const Plan &p, int rpt, void *scratch, cudaStream_t st) {
-  const int n = L.single.n;
+  const ScanDev &S = L.single;
+  const int n = S.n;
   float *copies = reinterpret_cast<float *>(scratch);
-  pack_single_kernel<<<dim3((n + 31) / 32, (n + 31) / 32), dim3(32, 8), 0, st>>>(L.single.buf[L.in_buf], copies, n);
+  pack_single_kernel<<<dim3((n + 31) / 32, (n + 31) / 32), dim3(32, 8), 0, st>>>(S.buf[L.in_buf], copies, n, S.lpitch,
+                                                                                 S.lpad);
   Launch Lt = L;
   Lt.single.pack = reinterpret_cast<float4 *>(copies);
   if (p.slab.ok) {
@@ -1129,15 +1369,17 @@ cudaError_t launch_fp_single(const Launch &L, const Plan &p, int rpt, void *scra
     CUtensorMap hmap;
     // (a descriptor the driver refuses reads as "not supported", a launch
     // configuration it refuses as "invalid argument")
-    if (encode_pack_tmap(&hmap, copies, n, 1, p.slab.wbox, p.slab.rows)) return cudaErrorNotSupported;
+    if (encode_pack_tmap(&hmap, copies, n, S.lpitch, 1, p.slab.wbox, p.slab.rows)) return cudaErrorNotSupported;
     cudaError_t e = cudaMemcpyAsync(dmap, &hmap, sizeof(hmap), cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return e;
     Lt.single.tmap = dmap;
     return launch_fp_slab(Lt, 1, p.slab.ncta, p.slab.views * p.slab.rays,
-                          slab_smem_bytes(1, p.slab.rows, p.slab.wbox), st);
+                          slab_smem_bytes(1, p.slab.rows, p.slab.wbox), st) < 0
+               ? cudaErrorInvalidValue
+               : cudaSuccess;
   }
   Lt.tr = 1;
-  return launch_fp(Lt, AT_GEOM_FAN, rpt, fp_ctas(L.single, rpt), st);
+  return launch_fp(Lt, AT_GEOM_FAN, rpt, fp_ctas(S, rpt), st);
 }
 
 // Forward projection of a batch of fan-beam / ray-table scans without groups:
@@ -1149,13 +1391,12 @@ int launch_fp_tr(const Launch &L, const Launch &Lpix, int rpt, int nctas, int pi
                  cudaStream_t st) {
   fp_pack_kernel<<<pix_nctas, 256, 0, st>>>(Lpix, 0);
   if (slab) {
-    if (launch_fp_slab(L, 1, nctas, slab->threads, slab->smem[1], st) != cudaSuccess) return -1;
-    return 2;
+    const int nl = launch_fp_slab(L, 1, nctas, slab->threads, slab->smem[1], st);
+    return nl < 0 ? -1 : 1 + nl;
   }
   Launch Lt = L;
   Lt.tr = 1;
-  launch_fp(Lt, AT_GEOM_FAN, rpt, nctas, st);
-  return 2;
+  return 1 + launch_fp_walk(Lt, rpt, nctas, st);
 }
 
 // Back projection of a batch whose scans sharing a plan are grouped: the max
@@ -1223,6 +1464,7 @@ int autotune_fan(Plan &p, cudaStream_t st) {
   p.fp_rpt = 1;
   free_slab_tables(p.slab);
   if (p.kind == AT_GEOM_GOLDNC || p.kind == AT_GEOM_CONE) return AT_OK;
+  if (p.line_ok) return AT_OK;  // one walk, faster than any of these
   float *img = nullptr, *sino = nullptr;
   void *scratch = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;

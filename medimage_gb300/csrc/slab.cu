@@ -34,6 +34,7 @@
 #include <vector>
 
 #include "epilogue.cuh"
+#include "line.cuh"
 #include "mbar.cuh"
 #include "solver.h"
 
@@ -60,54 +61,20 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, i
       : "memory");
 }
 
-template <int G>
-struct Elem;
-template <>
-struct Elem<1> {
-  using T = float;
-};
-template <>
-struct Elem<2> {
-  using T = float2;
-};
-template <>
-struct Elem<4> {
-  using T = float4;
-};
-
-template <int G>
-__device__ __forceinline__ void fma_elem(float (&part)[G], float wt, const typename Elem<G>::T &v) {
-  if constexpr (G == 1) {
-    part[0] = fmaf(wt, v, part[0]);
-  } else if constexpr (G == 2) {
-    part[0] = fmaf(wt, v.x, part[0]);
-    part[1] = fmaf(wt, v.y, part[1]);
-  } else {
-    part[0] = fmaf(wt, v.x, part[0]);
-    part[1] = fmaf(wt, v.y, part[1]);
-    part[2] = fmaf(wt, v.z, part[2]);
-    part[3] = fmaf(wt, v.w, part[3]);
-  }
-}
-
-template <int G>
-__device__ __forceinline__ typename Elem<G>::T zero_elem() {
-  if constexpr (G == 1) return 0.f;
-  else if constexpr (G == 2) return make_float2(0.f, 0.f);
-  else return make_float4(0.f, 0.f, 0.f, 0.f);
-}
-
 }  // namespace
 
 // G members per walk: 1 (a scan alone), 2 (a pair, float2) or 4 (three or four
-// members, float4).  Block = views x rays threads, one ray each.
-template <int G>
+// members, float4).  Block = views x rays threads, one ray each.  kLine: the
+// scans whose rays are lines (LineRay), walked row by row with the L1 walk's
+// operations (LineWalk); else the scans that walk decision bits.
+template <int G, bool kLine>
 __global__ void __launch_bounds__(512, 2) fan_fp_slab_kernel(const Launch L) {
   using T = typename Elem<G>::T;
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t *bar = reinterpret_cast<uint64_t *>(smem + ((8 - (smem_u32(smem) & 7u)) & 7u));
   const int scan = L.scans ? find_scan(L.prefix, L.nscans, blockIdx.x) : 0;
   const ScanDev &S = scan_of(L, scan);
+  if ((S.line != nullptr) != kLine) return;
   // the group's members and which of them this launch serves (read again for
   // the epilogue, so that they hold no registers through the walk)
   auto members = [&](const ScanDev *(&M)[G], bool(&act)[G]) {
@@ -137,7 +104,15 @@ __global__ void __launch_bounds__(512, 2) fan_fp_slab_kernel(const Launch L) {
   int nseg = 0, x0 = 0, y0 = 0, sx = 1, sy = 1;
   float ax = 0.f, ay = 0.f, lx = 0.f, ly = 0.f;
   const uint32_t *wp = S.bits;
-  if (valid) {
+  LineRay ray;
+  LineWalk<G> lw;
+  int lcol = 0, lcol0 = 0;  // kLine: the walked column, and where it began
+  LineTotal tot[G];
+  if constexpr (kLine) {
+    ray = valid ? load_line(S.line + (size_t)view * S.ndets + det) : line_none();
+    lw.load(ray);
+    lcol0 = line_c0(ray, S.n, S.lpitch);
+  } else if (valid) {
     const uint4 *hp = reinterpret_cast<const uint4 *>(S.rays + (size_t)view * S.ndets + det);
     const uint4 h0 = __ldg(hp), h1 = __ldg(hp + 1);
     nseg = (int)h0.y;
@@ -156,7 +131,24 @@ __global__ void __launch_bounds__(512, 2) fan_fp_slab_kernel(const Launch L) {
   for (int m = 0; m < G; m++) acc[m] = comp[m] = part[m] = 0.f;
   float cx = 0.f, cy = 0.f, prev = 0.f;
   const T *__restrict__ pack = reinterpret_cast<const T *>(S.pack);
-  if (flags & (kSlabFallback | kSlabEmpty)) {
+  if (kLine && (flags & (kSlabFallback | kSlabEmpty))) {
+    // gathers through L1 from the ray's own copy
+    if constexpr (kLine) {
+      const T *copy = pack + (ray.off - lcol0);
+      for (int r = lw.first & ~31; r <= lw.last; r++) {
+        if ((r & 31) == 0) lcol = lcol0 + lw.enter(r, S.n);
+        if (r < lw.first) {  // not in the grid yet
+          lcol += lw.crosses((float)(r & 31)) ? 1 : 0;
+          continue;
+        }
+        const T *row = copy + line_row_of(ray, r, S.n) * S.lpitch;
+        lcol += lw.row((float)(r & 31), __ldg(row + lcol), __ldg(row + lcol + 1)) ? 1 : 0;
+        if (r == lw.last || (r & 31) == 31)
+#pragma unroll
+          for (int m = 0; m < G; m++) tot[m].fold(lw.part[m]);
+      }
+    }
+  } else if (flags & (kSlabFallback | kSlabEmpty)) {
     // gathers through L1 from the row-major copy, with the L1 kernel's checks
     // (a pixel is read when its linear index lies in the image)
     const unsigned npix = (unsigned)(S.n * S.n);
@@ -201,7 +193,7 @@ __global__ void __launch_bounds__(512, 2) fan_fp_slab_kernel(const Launch L) {
       uint64_t *b = bar + (i & 1);
       mbar_expect_tx(b, box_bytes);
       void *dst = buf_base + (i & 1) * buf_bytes;
-      const int col = __ldg(wlo_row + s), row = row_base + s * SH;
+      const int col = __ldg(wlo_row + s) + S.lpad, row = row_base + s * SH;
       if constexpr (G == 4) tma_load_3d(dst, map, 0, col, row, b);
       else tma_load_2d(dst, map, col, row, b);
     };
@@ -228,7 +220,26 @@ __global__ void __launch_bounds__(512, 2) fan_fp_slab_kernel(const Launch L) {
     for (int i = 0; i < nsl; i++) {
       const int s = first + dir * i;
       if (!mbar_wait(bar + (i & 1), (unsigned)((i >> 1) & 1))) timed_out = true;
-      if (!timed_out && k < nseg && myslab == s) {
+      if constexpr (kLine) {
+        // the steps whose rows lie in the slab
+        const int u0 = s * SH, u1 = min(s * SH + SH, S.n) - 1;
+        const int r0 = max(dir > 0 ? u0 : S.n - 1 - u1, lw.first), r1 = min(dir > 0 ? u1 : S.n - 1 - u0, lw.last);
+        if (!timed_out && r0 <= r1) {
+          const T *tile = reinterpret_cast<const T *>(buf_base + (i & 1) * buf_bytes) -
+                          __ldg(wlo_row + s) + ((dir > 0 ? r0 : S.n - 1 - r0) - u0) * WB;
+          if (r0 == lw.first) {  // the block's steps before the grid
+            lcol = lcol0 + lw.enter(r0 & ~31, S.n);
+            for (int r = r0 & ~31; r < r0; r++) lcol += lw.crosses((float)(r & 31)) ? 1 : 0;
+          }
+          for (int r = r0; r <= r1; r++, tile += dir * WB) {
+            if ((r & 31) == 0) lcol = lcol0 + lw.enter(r, S.n);
+            lcol += lw.row((float)(r & 31), tile[lcol], tile[lcol + 1]) ? 1 : 0;
+            if (r == lw.last || (r & 31) == 31)
+#pragma unroll
+              for (int m = 0; m < G; m++) tot[m].fold(lw.part[m]);
+          }
+        }
+      } else if (!timed_out && k < nseg && myslab == s) {
         const T *tile = reinterpret_cast<const T *>(buf_base + (i & 1) * buf_bytes);
         const int row0 = s * SH;
         const int wlo = __ldg(wlo_row + s);
@@ -324,9 +335,20 @@ __global__ void __launch_bounds__(512, 2) fan_fp_slab_kernel(const Launch L) {
   for (int m = 0; m < G; m++) s0[m] = ff_zero();
   if (valid) {
     const int bin = view * S.ndets + det;
+    float out[G];
+    if constexpr (kLine) {
+#pragma unroll
+      for (int m = 0; m < G; m++)
+        out[m] = tot[m].finish(ray, S.lcorr, [&](int p) {
+          return __ldg(reinterpret_cast<const float *>(pack + (size_t)(p / S.n) * S.lpitch + S.lpad + p % S.n) + m);
+        });
+    } else {
+#pragma unroll
+      for (int m = 0; m < G; m++) out[m] = acc[m] - comp[m];
+    }
 #pragma unroll
     for (int m = 0; m < G; m++)
-      if (act[m]) fp_epilogue(*M[m], L, bin, acc[m] - comp[m], s0[m]);
+      if (act[m]) fp_epilogue(*M[m], L, bin, out[m], s0[m]);
   }
   if (stage_reduces(L.stage)) {
     if constexpr (G == 1) {
@@ -352,7 +374,7 @@ namespace {
 // Raises the kernel's dynamic shared memory limit to what a launch needs
 // (once per size; the limit is the device's opt-in maximum less the kernel's
 // static shared memory).  Returns cudaErrorInvalidValue for a size beyond it.
-template <int G>
+template <int G, bool kLine>
 cudaError_t launch_slab_g(const Launch &L, int nctas, int threads, size_t smem, cudaStream_t st) {
   static std::mutex mu;
   static size_t granted = 48 * 1024;  // every kernel may take 48 KB without opting in
@@ -363,40 +385,48 @@ cudaError_t launch_slab_g(const Launch &L, int nctas, int threads, size_t smem, 
       cudaError_t e = cudaGetDevice(&dev);
       if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
       cudaFuncAttributes fa{};
-      if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, fan_fp_slab_kernel<G>);
+      if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, fan_fp_slab_kernel<G, kLine>);
       if (e != cudaSuccess) return e;
       if (smem + fa.sharedSizeBytes > (size_t)optin) return cudaErrorInvalidValue;
-      e = cudaFuncSetAttribute(fan_fp_slab_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      e = cudaFuncSetAttribute(fan_fp_slab_kernel<G, kLine>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
       granted = smem;
     }
   }
-  fan_fp_slab_kernel<G><<<nctas, threads, smem, st>>>(L);
+  fan_fp_slab_kernel<G, kLine><<<nctas, threads, smem, st>>>(L);
   return cudaGetLastError();
+}
+
+template <int G>
+int launch_slab_forms(const Launch &L, int nctas, int threads, size_t smem, cudaStream_t st) {
+  const int forms = L.scans ? L.forms : L.single.line ? 2 : 1;
+  if ((forms & 2) && launch_slab_g<G, true>(L, nctas, threads, smem, st) != cudaSuccess) return -1;
+  if ((forms & 1) && launch_slab_g<G, false>(L, nctas, threads, smem, st) != cudaSuccess) return -1;
+  return forms == 3 ? 2 : 1;
 }
 }  // namespace
 
 // G: 1, 2 or 4 (the launch's group form).  The launch's scans share one CTA
 // shape (threads = views x rays); `smem` covers the largest slab buffer pair
-// among them.
-cudaError_t launch_fp_slab(const Launch &L, int G, int nctas, int threads, size_t smem, cudaStream_t st) {
-  if (nctas <= 0) return cudaSuccess;
-  if (G == 4) return launch_slab_g<4>(L, nctas, threads, smem, st);
-  if (G == 2) return launch_slab_g<2>(L, nctas, threads, smem, st);
-  return launch_slab_g<1>(L, nctas, threads, smem, st);
+// among them.  Returns the launches, or -1.
+int launch_fp_slab(const Launch &L, int G, int nctas, int threads, size_t smem, cudaStream_t st) {
+  if (nctas <= 0) return 0;
+  if (G == 4) return launch_slab_forms<4>(L, nctas, threads, smem, st);
+  if (G == 2) return launch_slab_forms<2>(L, nctas, threads, smem, st);
+  return launch_slab_forms<1>(L, nctas, threads, smem, st);
 }
 
 int slab_ctas(const ScanDev &S) {
   return ((S.nviews + S.slab_views - 1) / S.slab_views) * S.slab_ndb;
 }
 
-// TMA descriptor of a pack buffer: n x n pixels, row-major rows then the
-// transposed copy's rows (2n rows), G floats per pixel; box = the plan's slab
+// TMA descriptor of a pack buffer: rows of `pitch` pixels, the row-major copy's
+// n then the transposed copy's n, G floats per pixel; box = the plan's slab
 using EncodeTiledFn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                    const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                    CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-int encode_pack_tmap(CUtensorMap *out, const void *pack, int n, int G, int wbox, int rows) {
+int encode_pack_tmap(CUtensorMap *out, const void *pack, int n, int pitch, int G, int wbox, int rows) {
   static std::once_flag once;
   static EncodeTiledFn encode = nullptr;
   std::call_once(once, [] {
@@ -411,16 +441,16 @@ int encode_pack_tmap(CUtensorMap *out, const void *pack, int n, int G, int wbox,
   std::memset(out, 0, sizeof(*out));
   CUresult r;
   if (G == 4) {
-    const cuuint64_t dims[3] = {4, (cuuint64_t)n, 2 * (cuuint64_t)n};
-    const cuuint64_t strides[2] = {16, 16 * (cuuint64_t)n};
+    const cuuint64_t dims[3] = {4, (cuuint64_t)pitch, 2 * (cuuint64_t)n};
+    const cuuint64_t strides[2] = {16, 16 * (cuuint64_t)pitch};
     const cuuint32_t box[3] = {4, (cuuint32_t)wbox, (cuuint32_t)rows};
     const cuuint32_t es[3] = {1, 1, 1};
     r = encode(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void *>(pack), dims, strides, box, es,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   } else {
-    const cuuint64_t dims[2] = {(cuuint64_t)n, 2 * (cuuint64_t)n};
-    const cuuint64_t strides[1] = {(cuuint64_t)n * (G == 2 ? 8 : 4)};
+    const cuuint64_t dims[2] = {(cuuint64_t)pitch, 2 * (cuuint64_t)n};
+    const cuuint64_t strides[1] = {(cuuint64_t)pitch * (G == 2 ? 8 : 4)};
     const cuuint32_t box[2] = {(cuuint32_t)wbox, (cuuint32_t)rows};
     const cuuint32_t es[2] = {1, 1};
     r = encode(out, G == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
@@ -460,8 +490,9 @@ int check_wait_timeouts() {
 // CTA's middle that crosses the image (lenx > leny: the ray crosses more y
 // planes, so it runs closer to the y axis: the transposed copy), and the
 // direction of travel along that copy's rows.
+// Rays as lines have a direction of their own (LineRay).
 __global__ void slab_cta_kernel(int nviews, int ndets, int views, int rays, int ndb, int ncta, const RayHdr *hdr,
-                                unsigned *flags) {
+                                const LineRay *line, unsigned *flags) {
   const int cta = blockIdx.x * blockDim.x + threadIdx.x;
   if (cta >= ncta) return;
   const int vg = cta / ndb, db = cta % ndb;
@@ -472,6 +503,11 @@ __global__ void slab_cta_kernel(int nviews, int ndets, int views, int rays, int 
   for (int r = 0; r < (v1 - v0) * (d1 - d0) && (f & kSlabEmpty); r++) {
     const int v = v0 + (vm - v0 + r / (d1 - d0)) % (v1 - v0);
     const int d = d0 + (dm - d0 + r % (d1 - d0)) % (d1 - d0);
+    if (line) {
+      const LineRay l = line[(size_t)v * ndets + d];
+      if ((l.rows & 0xffffu) <= l.rows >> 16) f = ((l.flags & kLineSwap) ? kSlabTransposed : 0u) | ((l.flags & kLineDown) ? kSlabDown : 0u);
+      continue;
+    }
     const RayHdr h = hdr[(size_t)v * ndets + d];
     if (h.nseg == 0) continue;
     const bool tr = h.lenx > h.leny;
@@ -487,9 +523,42 @@ __global__ void slab_cta_kernel(int nviews, int ndets, int views, int rays, int 
 // rows against the CTA's direction.
 __global__ void slab_extent_kernel(int n, int nviews, int ndets, int nbpv, int views, int rays, int ndb, int rows,
                                    int nslab, const RayHdr *hdr, const uint32_t *bits, const uint32_t *blk_word,
-                                   const unsigned *flags, unsigned *fallback, int *lo, int *hi) {
+                                   const LineRay *line, const unsigned *flags, unsigned *fallback, int *lo,
+                                   int *hi) {
   const int ray = blockIdx.x * blockDim.x + threadIdx.x;
   if (ray >= nviews * ndets) return;
+  if (line) {  // every column the row walk reads, past the grid's edges too
+    const LineRay r = line[ray];
+    LineWalk<1> w;
+    w.load(r);
+    const int cta = (ray / ndets / views) * ndb + ray % ndets / rays;
+    if (w.empty()) return;
+    const unsigned mine = ((r.flags & kLineSwap) ? kSlabTransposed : 0u) | ((r.flags & kLineDown) ? kSlabDown : 0u);
+    if (mine != (flags[cta] & (kSlabTransposed | kSlabDown))) {
+      atomicOr(fallback + cta, 1u);
+      return;
+    }
+    const int col0 = line_c0(r, n, line_pitch(n));
+    int col = 0, mn = INT_MAX, mx = INT_MIN;
+    for (int k = w.first & ~31; k <= w.last; k++) {
+      if ((k & 31) == 0) col = col0 + w.enter(k, n);
+      if (k < w.first) {
+        col += w.crosses((float)(k & 31)) ? 1 : 0;
+        continue;
+      }
+      mn = min(mn, col);
+      mx = max(mx, col + 1);
+      col += w.row((float)(k & 31), 0.f, 0.f) ? 1 : 0;
+      const int u = line_row_of(r, k, n), next = (r.flags & kLineDown) ? u - 1 : u + 1;
+      if (k == w.last || next / rows != u / rows) {
+        atomicMin(lo + (size_t)cta * nslab + u / rows, mn);
+        atomicMax(hi + (size_t)cta * nslab + u / rows, mx);
+        mn = INT_MAX;
+        mx = INT_MIN;
+      }
+    }
+    return;
+  }
   const RayHdr h = hdr[ray];
   if (h.nseg == 0) return;
   const int view = ray / ndets, det = ray % ndets;
@@ -574,13 +643,14 @@ int build_slab_tables(Plan &p, int views, int rays, int rows, cudaStream_t st) {
   AT_CUDA_TRY(cudaMalloc(&hi, sizeof(int) * cells));
   AT_CUDA_TRY(cudaMemsetAsync(fb, 0, sizeof(unsigned) * ncta, st));
   AT_CUDA_TRY(cudaMemsetAsync(lo, 0x7f, sizeof(int) * cells, st));  // 0x7f7f7f7f: above any column
-  AT_CUDA_TRY(cudaMemsetAsync(hi, 0xff, sizeof(int) * cells, st));  // -1: below any column
-  slab_cta_kernel<<<(ncta + 127) / 128, 128, 0, st>>>(nviews, ndets, views, rays, ndb, ncta, p.rays_d, flags);
+  AT_CUDA_TRY(cudaMemsetAsync(hi, 0x80, sizeof(int) * cells, st));  // 0x80808080: below any column
+  slab_cta_kernel<<<(ncta + 127) / 128, 128, 0, st>>>(nviews, ndets, views, rays, ndb, ncta, p.rays_d,
+                                                    p.line_ok ? p.line_d : nullptr, flags);
   AT_CUDA_TRY(cudaGetLastError());
   const int nrays = nviews * ndets;
   slab_extent_kernel<<<(nrays + 127) / 128, 128, 0, st>>>(n, nviews, ndets, p.nblocks_per_view, views, rays, ndb,
-                                                         rows, nslab, p.rays_d, p.bits_d, p.blk_word_d, flags, fb,
-                                                         lo, hi);
+                                                         rows, nslab, p.rays_d, p.bits_d, p.blk_word_d,
+                                                         p.line_ok ? p.line_d : nullptr, flags, fb, lo, hi);
   AT_CUDA_TRY(cudaGetLastError());
   std::vector<unsigned> hf(ncta), hfb(ncta);
   std::vector<int> hlo(cells), hhi(cells);

@@ -29,7 +29,7 @@ int launch_fp_tr(const Launch &L, const Launch &Lpix, int rpt, int nctas, int pi
 int slab_ctas(const ScanDev &S);
 int cone_bp_launches(int chunks);
 size_t slab_smem_bytes(int G, int rows, int wbox);
-int encode_pack_tmap(CUtensorMap *out, const void *pack, int n, int G, int wbox, int rows);
+int encode_pack_tmap(CUtensorMap *out, const void *pack, int n, int pitch, int G, int wbox, int rows);
 int launch_bp_group(const Launch &L, const Launch &Lsino, const Launch &Lsmall, int nctas, int sino_nctas,
                     int small_nctas, cudaStream_t st);
 cudaError_t launch_bp(const Launch &L, int kind, int nctas, cudaStream_t st, const Launch *Lpix, int pix_nctas);
@@ -51,6 +51,10 @@ void fill_scan_plan(ScanDev &S, const Plan &p) {
   S.bits = p.bits_d;
   S.blk_word = p.blk_word_d;
   S.blk_off = p.blk_off_d;
+  S.line = p.line_ok ? p.line_d : nullptr;
+  S.lcorr = p.lcorr_d;
+  S.lpitch = p.line_ok ? line_pitch(p.n) : p.n;
+  S.lpad = p.line_ok ? kLinePad : 0;
   S.run = p.run_d;
   S.tile_off = p.tile_off_d;
   S.pt_meta = p.pt_meta_d;
@@ -92,6 +96,14 @@ enum PixKernel { PK_UPD = 0, PK_PP, PK_COMMIT, PK_EDGE_INIT, PK_EDGE_D, PK_EDGE_
 
 size_t align_up(size_t x) { return (x + 255) & ~size_t(255); }
 
+// a fan-beam / ray-table scan's pack buffer: a group's images, row-major and
+// transposed, or its sinograms, interleaved
+size_t pack_bytes_of(const Plan &p) {
+  if (p.kind != AT_GEOM_FAN && p.kind != AT_GEOM_RAYS) return 0;
+  const size_t copies = 2 * (size_t)p.n * (p.line_ok ? line_pitch(p.n) : p.n);
+  return align_up(sizeof(float4) * std::max(copies, (size_t)p.nviews * p.ndets));
+}
+
 struct ScanLayout {
   size_t img_bytes, sino_bytes, partial_bytes, trace_bytes, bp_bytes, pack_bytes, total;
 };
@@ -110,10 +122,7 @@ ScanLayout layout_of(const Plan &p, int rpt) {
   L.partial_bytes = align_up((size_t)maxcta * 4 * sizeof(double));
   L.trace_bytes = align_up((size_t)kTraceCap * 10 * sizeof(double));
   L.bp_bytes = bp_scratch_bytes(p);
-  // fan beam and ray tables: a group's forward-projector inputs, interleaved
-  const bool packs = p.kind == AT_GEOM_FAN || p.kind == AT_GEOM_RAYS;
-  // (images twice: row-major and transposed)
-  L.pack_bytes = packs ? align_up(sizeof(float4) * std::max(2 * (size_t)p.n * p.n, nbins)) : 0;
+  L.pack_bytes = pack_bytes_of(p);
   L.total = L.img_bytes * B_NIMG + L.sino_bytes * (B_NBUF - B_NIMG) + L.partial_bytes + L.trace_bytes +
             L.bp_bytes + L.pack_bytes + align_up(sizeof(Ctl));
   return L;
@@ -259,12 +268,14 @@ int Batch::set(const ScanDev *scans, int n, int kind_, int rpt_, cudaStream_t st
       slab_launch.smem[form] = std::max(slab_launch.smem[form], slab_smem_bytes(G, S.slab_rows, S.slab_wbox));
       S.tmap = tmaps_d + s;
       if (S.nmem == 0) continue;  // a member: its lead's walk reads the group's pack buffer
-      int rc = encode_pack_tmap(&maps[s], S.pack, S.n, G, S.slab_wbox, S.slab_rows);
+      int rc = encode_pack_tmap(&maps[s], S.pack, S.n, S.lpitch, G, S.slab_wbox, S.slab_rows);
       if (rc) return rc;
     }
     AT_CUDA_TRY(cudaMemcpyAsync(tmaps_d, maps.data(), sizeof(CUtensorMap) * n, cudaMemcpyHostToDevice, st));
   }
   scans = sc.data();
+  forms = 0;
+  for (const auto &S : sc) forms |= S.line ? 2 : 1;
   cone_chunks = 1;
   for (const auto &S : sc)
     if (S.kind == AT_GEOM_CONE) cone_chunks = std::max(cone_chunks, (S.nviews + S.bp_vchunk - 1) / std::max(1, S.bp_vchunk));
@@ -373,6 +384,7 @@ Launch Batch::base_launch(int family) const {
   L.aux_buf = -1;
   L.group = (family == FAM_PIX || family == FAM_SINO) ? 1 : group;
   L.chunks = cone_chunks;
+  L.forms = forms;
   const bool fp = family == FAM_FP || family == FAM_FP1 || family == FAM_FP2;
   if (persistent && (family == FAM_BP || family == FAM_BPS || (fp && !slab))) {
     L.queue = queue_d;
@@ -590,12 +602,8 @@ int ProjSet::create(const std::vector<Plan *> &pl) {
   plans = pl;
   rpt = Solver::choose_rpt(pl);
   const int n = (int)pl.size();
-  auto pack_of = [](const Plan &p) {
-    const size_t elems = std::max(2 * (size_t)p.n * p.n, (size_t)p.nviews * p.ndets);
-    return (p.kind == AT_GEOM_FAN || p.kind == AT_GEOM_RAYS) ? align_up(sizeof(float4) * elems) : 0;
-  };
   size_t total = 256;
-  for (auto *p : pl) total += bp_scratch_bytes(*p) + pack_of(*p);
+  for (auto *p : pl) total += bp_scratch_bytes(*p) + pack_bytes_of(*p);
   if (cudaMalloc(&scratch, total) != cudaSuccess) {
     cudaGetLastError();
     return set_error(AT_ENOMEM, "projection set: device allocation of " + std::to_string(total) + " bytes failed");
@@ -608,8 +616,8 @@ int ProjSet::create(const std::vector<Plan *> &pl) {
     fill_scan_plan(host[s], *pl[s]);
     carve_bp_scratch(host[s], *pl[s], cur);
     cur += bp_scratch_bytes(*pl[s]);
-    host[s].pack = pack_of(*pl[s]) ? (float4 *)cur : nullptr;
-    cur += pack_of(*pl[s]);
+    host[s].pack = pack_bytes_of(*pl[s]) ? (float4 *)cur : nullptr;
+    cur += pack_bytes_of(*pl[s]);
   }
   return AT_OK;
 }

@@ -92,6 +92,9 @@ struct ScanDev {
   const uint32_t *bits;
   const uint32_t *blk_word;
   const uint8_t *blk_off;  // per 128-ray block: a ray leaves the grid
+  const LineRay *line;     // the rays as lines (null: walk the decision bits)
+  const LineCorr *lcorr;
+  int lpitch, lpad;        // row pitch and first column of the pack buffer's image copies
   const uint4 *run;          // back-projection runs grouped by 16x16 tile
   const int32_t *tile_off;   // [tile * nvb + view block]
   // the plan's pixel table (Plan::pt_*), and which launches gather from it
@@ -156,6 +159,7 @@ struct Launch {
   int chunks;                    // cone back projection: chunks of the launch's largest scan (host side)
   int group;                     // projector launches: largest group of scans sharing a plan
   int tr;                        // forward projection: the scans' pack buffers hold transposed inputs
+  int forms;                     // fan projectors (host side): 1 some scans walk bits, 2 some walk lines
   int bp_table;                  // fan back projection: 0 walk tile runs, 1 gather from pixel tables,
                                  // 2 each CTA as its scan's plan says (ScanDev::pt_use)
   // persistent launches (projectors of a batch): a grid sized to the resident
