@@ -80,6 +80,16 @@ constexpr int32_t kCorrForwardOnly = 1 << 30;
 // rows transposed.  A walk strays at most two columns past the grid.
 constexpr int kLinePad = 4;
 constexpr int line_pitch(int n) { return (n + 2 * kLinePad + 3) & ~3; }
+// The back projector along lines (strip.cu) takes strips of whole cells of
+// kStripCellRows rows and kStripCellCols columns, and one of several
+// divisions of the views (a launch chooses).
+constexpr int kStripCellRows = 16, kStripCellCols = 128;
+constexpr int kStripDivs = 16;
+struct __align__(16) StripCorr {  // a ray's correction (LineCorr)
+  int32_t ray, pix;
+  float w;
+  int32_t pad;
+};
 
 struct GcSeg {   // one GoldenC walk segment
   int32_t pix;   // Y*512 + X (tile-global, symmetry 0 frame)
@@ -146,6 +156,17 @@ struct Plan {
   LineRay *line_d = nullptr;
   LineCorr *lcorr_d = nullptr;
   int64_t ncorr = 0;
+  // back projection along the lines (strip.cu), the default where there are
+  // lines: per view, direction (rows along x or y) and cell the first and last
+  // detector whose ray meets the cell; the ranges of views a CTA takes,
+  // {first << 1 | direction, views}, of division q from strip_poff[q]; the rays'
+  // corrections; detectors between a warp's rays
+  int strip_ok = 0;
+  int2 *strip_rng_d = nullptr;
+  int2 *strip_part_d = nullptr;
+  int strip_poff[kStripDivs + 1] = {};
+  StripCorr *strip_corr_d = nullptr;
+  int strip_ncr = 0, strip_ncc = 0, strip_k = 1, strip_ncorr = 0;
   // back projection: one entry per (ray, 16x16 tile) run of the traversal,
   // grouped by tile, longest runs first.  Entry = {ray, k_in | nk << 14 |
   // cx_in << 19, the run's decision bits (bit j = segment k_in + j; a run in a
@@ -173,6 +194,7 @@ struct Plan {
   int64_t *pt_woff_d = nullptr;
   int64_t pt_entries = 0, pt_bytes = 0;
   int bp_table = 0;  // launches that back-project from the table: bit0 single scans, bit1 groups
+  int bp_pinned = 0; // at_plan_set_back_variant chose: tile runs or the table, never strips
   // goldnc
   GcSeg *gc_seg_d = nullptr;
   int32_t *gc_pair_off_d = nullptr;  // [17280+1]
@@ -229,6 +251,8 @@ void retire_slab_tables(Plan &p);  // moves p.slab to p.retired_slabs
 // pixels in one view) or the table would exceed max_bytes
 int build_pixel_table(Plan &p, int64_t max_bytes, cudaStream_t st);
 void free_pixel_table(Plan &p);
+// tables of the back projector along lines (strip.cu)
+int build_strips(Plan &p, const std::vector<int> &off, const std::vector<LineCorr> &corr, cudaStream_t st);
 // AT_ECUDA when a bounded wait of the slab projector ran out since the last
 // call (its CTAs' outputs are void); called after a synchronisation
 int check_wait_timeouts();

@@ -19,6 +19,7 @@ cudaError_t launch_fp_single(const Launch &L, const Plan &p, int rpt, void *scra
 size_t fp_single_scratch_bytes(const Plan &p);
 int bp_ctas(const ScanDev &S);
 cudaError_t launch_fp(const Launch &L, int kind, int rpt, int nctas, cudaStream_t st);
+void strip_choose(ScanDev *scans, int n);
 cudaError_t launch_bp(const Launch &L, int kind, int nctas, cudaStream_t st, const Launch *Lpix, int pix_nctas);
 int pix_ctas(const ScanDev &S);
 cudaError_t launch_median(const float *in, float *out, int n, cudaStream_t st);
@@ -79,12 +80,15 @@ int project(const Plan &p, bool forward, const float *in, float *out, cudaStream
     void *scratch = nullptr;
     if (bpb) {
       AT_CUDA_TRY(cudaMallocAsync(&scratch, bpb, st));
-      if ((e = cudaMemsetAsync(scratch, 0, bpb, st)) != cudaSuccess) {
+      // (scratch that strips use is cleared by their first kernel)
+      if (!L.single.strip && (e = cudaMemsetAsync(scratch, 0, bpb, st)) != cudaSuccess) {
         cudaFreeAsync(scratch, st);
         return cuda_error(e, "back projection scratch");
       }
       carve_bp_scratch(L.single, p, (char *)scratch);
       L.single.bp_split = bp_split_for(p.ntiles, p.nvb);
+      L.single.nmem = 1;
+      strip_choose(&L.single, 1);
     }
     L.bp_table = (L.single.pt_use & 1) ? 1 : 0;
     if (p.kind == AT_GEOM_CONE) L.chunks = (p.nviews + p.cone_bp_views - 1) / std::max(1, p.cone_bp_views);
@@ -260,6 +264,7 @@ AT_API int at_plan_set_back_variant(at_plan *plan, int32_t use) {
     if (!p.pt_meta_d) return set_error(AT_EINVAL, "at_plan_set_back_variant: the pixel table does not fit this plan");
   }
   p.bp_table = use;
+  p.bp_pinned = 1;
   return AT_OK;
 }
 

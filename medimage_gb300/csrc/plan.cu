@@ -624,7 +624,10 @@ int build_lines(Plan &p, const RaySource &R, cudaStream_t st) {
   p.device_bytes += (int64_t)sizeof(LineRay) * nrays;
   p.ncorr = tot;
   p.line_ok = 1;
-  return AT_OK;
+  std::vector<LineCorr> corr((size_t)tot);
+  if (tot) AT_CUDA_TRY(cudaMemcpyAsync(corr.data(), p.lcorr_d, sizeof(LineCorr) * tot, cudaMemcpyDeviceToHost, st));
+  AT_CUDA_TRY(cudaStreamSynchronize(st));
+  return build_strips(p, off, corr, st);
 }
 
 int build_fan_plan(Plan &p, cudaStream_t st, const double *h_ends) {
@@ -951,6 +954,9 @@ Plan::~Plan() {
   cudaFree(blk_off_d);
   cudaFree(line_d);
   cudaFree(lcorr_d);
+  cudaFree(strip_rng_d);
+  cudaFree(strip_part_d);
+  cudaFree(strip_corr_d);
   cudaFree(run_d);
   cudaFree(tile_off_d);
   cudaFree(gc_seg_d);

@@ -613,13 +613,23 @@ constexpr int bp_copy_stride() {
 
 // max |r| of each scan's input sinogram, in kBpMaxParts partial maxima
 __global__ void __launch_bounds__(256) sino_absmax_kernel(const Launch L) {
+  asm volatile("griddepcontrol.launch_dependents;");  // strip_bp_kernel prepares meanwhile
   const int scan = blockIdx.x / kBpMaxParts, part = blockIdx.x % kBpMaxParts;
   const ScanDev &S = scan_of(L, L.scans ? scan : 0);
   if (!flow_active(S, L.flow)) return;
   const float *__restrict__ sino = S.buf[L.in_buf];
   float m = 0.f;
-  for (int i = part * blockDim.x + threadIdx.x; i < S.nbins; i += kBpMaxParts * blockDim.x)
-    m = fmaxf(m, fabsf(__ldg(sino + i)));
+  const int step = kBpMaxParts * blockDim.x;
+  int i = part * blockDim.x + threadIdx.x;
+  // eight loads in flight: the pass is their latency (C2: 20 -> X us)
+  for (; i + 7 * step < S.nbins; i += 8 * step) {
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) v[j] = __ldg(sino + i + j * step);
+#pragma unroll
+    for (int j = 0; j < 8; j++) m = fmaxf(m, fabsf(v[j]));
+  }
+  for (; i < S.nbins; i += step) m = fmaxf(m, fabsf(__ldg(sino + i)));
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
   __shared__ float wm[8];
@@ -629,6 +639,9 @@ __global__ void __launch_bounds__(256) sino_absmax_kernel(const Launch L) {
     for (int w = 1; w < (int)(blockDim.x >> 5); w++) m = fmaxf(m, wm[w]);
     S.bpmax[part] = m;
   }
+  // fresh scratch: its sums start at zero
+  if (L.flag)
+    for (int i = part * blockDim.x + threadIdx.x; i < S.npix; i += step) S.bp_acc[i] = 0ull;
 }
 
 // v added to the shared-memory word *p as a reduction (PTX red: no value
@@ -782,6 +795,7 @@ __device__ __forceinline__ void fan_bp_body(const Launch &L, const int unit) {
   constexpr int kMemStride = C * kStride;       // one member
   const int scan = L.scans ? find_scan(L.prefix, L.nscans, unit) : 0;
   const ScanDev &S = scan_of(L, scan);
+  if (S.strip) return;  // strip_bp_kernel's
   const int nm = L.scans ? S.nmem : 1;
   const ScanDev *M[G];
   bool act[G];
@@ -1160,6 +1174,9 @@ int launch_fp_slab(const Launch &L, int G, int nctas, int threads, size_t smem, 
 size_t slab_smem_bytes(int G, int rows, int wbox);
 int encode_pack_tmap(CUtensorMap *out, const void *pack, int n, int pitch, int G, int wbox, int rows);
 cudaError_t launch_cone_bp(const Launch &L, int nctas, const Launch &Lpix, int pix_nctas, cudaStream_t st);
+int strip_ctas(const ScanDev &S);
+cudaError_t launch_strip_bp(const Launch &L, int nctas, cudaStream_t st);
+cudaError_t launch_strip_finish(const Launch &Lpix, int pix_nctas, cudaStream_t st);
 
 // CTAs of `kernel` (with `threads` threads) resident on the whole device at
 // once: the grid of its persistent (queue) form
@@ -1216,6 +1233,7 @@ int cone_bp_ctas(const ScanDev &S);
 int bp_ctas(const ScanDev &S) {
   if (S.kind == AT_GEOM_GOLDNC) return (kGcN / 8) * (kGcN / 32);
   if (S.kind == AT_GEOM_CONE) return cone_bp_ctas(S);
+  if (S.strip) return strip_ctas(S);
   return S.ntiles_y * S.ntiles_y * std::max(1, S.bp_split);
 }
 
@@ -1401,11 +1419,14 @@ int launch_fp_tr(const Launch &L, const Launch &Lpix, int rpt, int nctas, int pi
 
 // Back projection of a batch whose scans sharing a plan are grouped: the max
 // |r| pass, the members' sinograms interleaved (over the sinogram-pass CTAs
-// of Lsino), then each group's runs walked once: groups of three or four over
-// L's CTAs, pairs and scans alone over Lsmall's.  Returns the number of
-// launches.
-int launch_bp_group(const Launch &L, const Launch &Lsino, const Launch &Lsmall, int nctas, int sino_nctas,
-                    int small_nctas, cudaStream_t st) {
+// of Lsino), then each group's rays walked once: groups of three or four over
+// L's CTAs, pairs and scans alone over Lsmall's; by strips (and their per-pixel
+// pass, over Lpix's) for plans with lines, by tile runs or tables for the
+// others.  L's CTAs are those of the larger groups and of every scan or group
+// that goes by strips (the two kernels' CTAs of the other's return at once),
+// Lsmall's the rest.  Returns the number of launches, or -1.
+int launch_bp_group(const Launch &L, const Launch &Lsino, const Launch &Lsmall, const Launch &Lpix, int nctas,
+                    int sino_nctas, int small_nctas, int pix_nctas, cudaStream_t st) {
   int n = 2;
   Launch La = L;  // the max |r| pass: one CTA per part, never queued
   La.queue = nullptr;
@@ -1418,13 +1439,21 @@ int launch_bp_group(const Launch &L, const Launch &Lsino, const Launch &Lsmall, 
   auto small = [&](auto kern, int m) {
     launch_maybe_queued(kern, fan_bp_small_queue_kernel, ress[m], Lsmall, small_nctas, 256, st);
   };
-  if (L.bp_table == 1) group(fan_bp_group_kernel<1>, 1);
-  else if (L.bp_table == 2) group(fan_bp_group_kernel<2>, 2);
-  else group(fan_bp_group_kernel<0>, 0);
-  if (Lsmall.bp_table == 1) small(fan_bp_small_kernel<1>, 1);
-  else if (Lsmall.bp_table == 2) small(fan_bp_small_kernel<2>, 2);
-  else small(fan_bp_small_kernel<0>, 0);
-  return n + (nctas > 0) + (small_nctas > 0);
+  if (L.bp_forms & 4) {
+    n++;
+    if (L.bp_table == 1) group(fan_bp_group_kernel<1>, 1);
+    else if (L.bp_table == 2) group(fan_bp_group_kernel<2>, 2);
+    else group(fan_bp_group_kernel<0>, 0);
+  }
+  if (L.bp_forms & 3) {
+    n++;
+    if (Lsmall.bp_table == 1) small(fan_bp_small_kernel<1>, 1);
+    else if (Lsmall.bp_table == 2) small(fan_bp_small_kernel<2>, 2);
+    else small(fan_bp_small_kernel<0>, 0);
+  }
+  if (!(L.bp_forms & 56)) return n;
+  if (launch_strip_bp(L, nctas, st) != cudaSuccess) return -1;
+  return launch_strip_finish(Lpix, pix_nctas, st) == cudaSuccess ? n + 2 : -1;
 }
 
 // Lpix / pix_nctas: the same launch over pixel-pass CTAs, for kernels whose
@@ -1439,7 +1468,15 @@ cudaError_t launch_bp(const Launch &L, int kind, int nctas, cudaStream_t st, con
   } else {
     Launch La = L;  // the max |r| pass: one CTA per part, never queued
     La.queue = nullptr;
+    const int forms = L.scans ? L.bp_forms : L.single.strip ? 8 : 1;
+    La.flag = !L.scans && forms == 8;
     sino_absmax_kernel<<<(L.scans ? L.nscans : 1) * kBpMaxParts, 256, 0, st>>>(La);
+    if (forms & 56) {
+      if (!Lpix) return cudaErrorInvalidValue;
+      cudaError_t e = launch_strip_bp(L, nctas, st);
+      if (e == cudaSuccess) e = launch_strip_finish(*Lpix, pix_nctas, st);
+      if (e != cudaSuccess || !(forms & 7)) return e;
+    }
     static int res[3] = {0, 0, 0};
     if (L.bp_table == 1) launch_maybe_queued(fan_bp_kernel<1>, fan_bp_queue_kernel, res[1], L, nctas, 256, st);
     else if (L.bp_table == 2) launch_maybe_queued(fan_bp_kernel<2>, fan_bp_queue_kernel, res[2], L, nctas, 256, st);

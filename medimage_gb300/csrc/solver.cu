@@ -30,8 +30,9 @@ int slab_ctas(const ScanDev &S);
 int cone_bp_launches(int chunks);
 size_t slab_smem_bytes(int G, int rows, int wbox);
 int encode_pack_tmap(CUtensorMap *out, const void *pack, int n, int pitch, int G, int wbox, int rows);
-int launch_bp_group(const Launch &L, const Launch &Lsino, const Launch &Lsmall, int nctas, int sino_nctas,
-                    int small_nctas, cudaStream_t st);
+int launch_bp_group(const Launch &L, const Launch &Lsino, const Launch &Lsmall, const Launch &Lpix, int nctas,
+                    int sino_nctas, int small_nctas, int pix_nctas, cudaStream_t st);
+void strip_choose(ScanDev *scans, int n);
 cudaError_t launch_bp(const Launch &L, int kind, int nctas, cudaStream_t st, const Launch *Lpix, int pix_nctas);
 cudaError_t launch_pixel(int which, const Launch &L, int nctas, cudaStream_t st);
 cudaError_t launch_flags(const ScanDev *scans, int nscans, int mode, cudaStream_t st);
@@ -61,6 +62,15 @@ void fill_scan_plan(ScanDev &S, const Plan &p) {
   S.pt_w = p.pt_w_d;
   S.pt_woff = p.pt_woff_d;
   S.pt_use = p.pt_meta_d ? p.bp_table : 0;
+  S.strip = p.strip_ok && !p.bp_pinned ? 1 : 0;
+  S.strip_ncr = p.strip_ncr;
+  S.strip_ncc = p.strip_ncc;
+  S.strip_k = p.strip_k;
+  std::copy(std::begin(p.strip_poff), std::end(p.strip_poff), S.strip_poff);
+  S.strip_rng = p.strip_rng_d;
+  S.strip_part0 = p.strip_part_d;
+  S.strip_ncorr = p.strip_ncorr;
+  S.strip_corr = p.strip_corr_d;
   S.ntiles_y = p.ntiles_y;
   S.nvb = p.nvb;
   S.bp_term_bits = p.bp_term_bits;
@@ -250,6 +260,7 @@ int Batch::set(const ScanDev *scans, int n, int kind_, int rpt_, cudaStream_t st
     }
     const int split = bp_split_for(tiles, nvb);
     for (auto &S : sc) S.bp_split = split;
+    strip_choose(sc.data(), n);
   }
   // the slab forward projector, when every plan has slab tables of one CTA
   // shape: each lead's TMA descriptor covers its pack buffer in its group's
@@ -274,8 +285,11 @@ int Batch::set(const ScanDev *scans, int n, int kind_, int rpt_, cudaStream_t st
     AT_CUDA_TRY(cudaMemcpyAsync(tmaps_d, maps.data(), sizeof(CUtensorMap) * n, cudaMemcpyHostToDevice, st));
   }
   scans = sc.data();
-  forms = 0;
-  for (const auto &S : sc) forms |= S.line ? 2 : 1;
+  forms = bp_forms = 0;
+  for (const auto &S : sc) {
+    forms |= S.line ? 2 : 1;
+    if (S.nmem) bp_forms |= (S.strip ? 8 : 1) << (S.nmem >= 3 ? 2 : S.nmem - 1);
+  }
   cone_chunks = 1;
   for (const auto &S : sc)
     if (S.kind == AT_GEOM_CONE) cone_chunks = std::max(cone_chunks, (S.nviews + S.bp_vchunk - 1) / std::max(1, S.bp_vchunk));
@@ -291,8 +305,9 @@ int Batch::set(const ScanDev *scans, int n, int kind_, int rpt_, cudaStream_t st
       add(FAM_FP, s, big ? fpc : 0);
       add(FAM_FP1, s, nm == 1 ? fpc : 0);
       add(FAM_FP2, s, nm == 2 ? fpc : 0);
-      add(FAM_BP, s, big ? bp_ctas(scans[s]) : 0);
-      add(FAM_BPS, s, small ? bp_ctas(scans[s]) : 0);
+      const bool strip = scans[s].strip != 0;  // one launch for all
+      add(FAM_BP, s, big || (small && strip) ? bp_ctas(scans[s]) : 0);
+      add(FAM_BPS, s, small && !strip ? bp_ctas(scans[s]) : 0);
     } else {
       add(FAM_FP, s, slab ? slab_ctas(scans[s]) : fp_ctas(scans[s], rpt));
       add(FAM_FP1, s, 0);
@@ -385,6 +400,7 @@ Launch Batch::base_launch(int family) const {
   L.group = (family == FAM_PIX || family == FAM_SINO) ? 1 : group;
   L.chunks = cone_chunks;
   L.forms = forms;
+  L.bp_forms = bp_forms;
   const bool fp = family == FAM_FP || family == FAM_FP1 || family == FAM_FP2;
   if (persistent && (family == FAM_BP || family == FAM_BPS || (fp && !slab))) {
     L.queue = queue_d;
@@ -422,16 +438,19 @@ int Batch::enqueue_bp(const Launch &L, cudaStream_t st) {
     Launch Lb = L, Lsm = retarget(L, FAM_BPS);
     Lb.bp_table = bp_table_main;
     Lsm.bp_table = bp_table_small;
-    launches += launch_bp_group(Lb, Ls, Lsm, bp_total, sino_total, bps_total, st);
+    const int nl = launch_bp_group(Lb, Ls, Lsm, retarget(L, FAM_PIX), bp_total, sino_total, bps_total, pix_total, st);
     AT_CUDA_TRY(cudaGetLastError());
+    if (nl < 0) return set_error(AT_ECUDA, "grouped back projection launch failed");
+    launches += nl;
     return AT_OK;
   }
-  const Launch Lp = retarget(L, FAM_PIX);  // the per-pixel finishing pass of the cone-beam back projector
+  const Launch Lp = retarget(L, FAM_PIX);  // the per-pixel finishing pass (cone beam, strips)
   Launch Lb = L;
   Lb.bp_table = bp_table_main;
   AT_CUDA_TRY(launch_bp(Lb, kind, bp_total, st, &Lp, pix_total));
   // max |r| pass + back projection (cone beam: its chunks, folds and per-pixel finish)
-  launches += kind == AT_GEOM_GOLDNC ? 1 : kind == AT_GEOM_CONE ? cone_bp_launches(cone_chunks) : 2;
+  launches += kind == AT_GEOM_GOLDNC ? 1 : kind == AT_GEOM_CONE ? cone_bp_launches(cone_chunks)
+                                          : 1 + (bp_forms & 7 ? 1 : 0) + (bp_forms & 56 ? 2 : 0);
   return AT_OK;
 }
 

@@ -103,6 +103,13 @@ struct ScanDev {
   const float *pt_w;
   const int64_t *pt_woff;
   int pt_use;
+  // back projection along lines (Plan::strip_*): 0 for tile runs or the table;
+  // strip_parts: the strip_npart ranges of views of the launch
+  int strip, strip_ncr, strip_ncc, strip_k, strip_npart, strip_ncorr;
+  int strip_poff[kStripDivs + 1];
+  const int2 *strip_rng;
+  const int2 *strip_part0, *strip_parts;
+  const StripCorr *strip_corr;
   int ntiles_y, nvb, bp_term_bits;
   float pixel_mm;
   // goldnc plan
@@ -160,6 +167,8 @@ struct Launch {
   int group;                     // projector launches: largest group of scans sharing a plan
   int tr;                        // forward projection: the scans' pack buffers hold transposed inputs
   int forms;                     // fan projectors (host side): 1 some scans walk bits, 2 some walk lines
+  int bp_forms;                  // fan back projection (host side): bits 0..2 some scans alone / pairs / larger
+                                 // groups walk tile runs or gather from the table, bits 3..5 some walk strips
   int bp_table;                  // fan back projection: 0 walk tile runs, 1 gather from pixel tables,
                                  // 2 each CTA as its scan's plan says (ScanDev::pt_use)
   // persistent launches (projectors of a batch): a grid sized to the resident

@@ -445,9 +445,10 @@ class Plan:
         self.stats = {k: getattr(st, k) for k, _ in _PlanStats._fields_}
 
     def set_back_variant(self, use: int) -> None:
-        """Back projector of later batches: bit0 single scans, bit1 groups of
-        scans sharing the plan gather from the pixel table (built on first
-        use); a clear bit walks tile runs.  Bitwise the same sums."""
+        """Pin the back projector of later batches (by default rays are walked
+        as lines): bit0 single scans, bit1 groups of scans sharing the plan
+        gather from the pixel table (built on first use); a clear bit walks
+        tile runs.  Bitwise the same sums either way."""
         _check("at_plan_set_back_variant", lib().at_plan_set_back_variant(self._h, use))
         st = _PlanStats()
         _check("at_plan_get_stats", lib().at_plan_get_stats(self._h, C.byref(st)))
