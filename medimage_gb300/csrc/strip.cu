@@ -182,14 +182,8 @@ __device__ __forceinline__ void strip_bp_body(const Launch &L, const int scan, c
   constexpr int kCellRows = kRows / kStripCellRows;
   static_assert(kRows % kStripCellRows == 0 && StripShape<G>::cols % kStripCellCols == 0, "strips are whole cells");
   __shared__ float s_max[G];
-  const int nm = L.scans ? S.nmem : 1;
   const int n = S.n, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  unsigned act = 0;
-#pragma unroll
-  for (int m = 0; m < G; m++) {
-    const ScanDev &M = L.scans ? L.scans[S.mem[m < nm ? m : 0]] : L.single;
-    if (m < nm && flow_active(M, L.flow)) act |= 1u << m;
-  }
+  const unsigned act = group_active<G>(L, S);
   if (!act) return grid_dependency_wait();
   // this CTA's views, direction and strip
   const int tcells = strip_tile_cells(S.strip_ncc, StripShape<G>::cols), ntile = (S.strip_ncc + tcells - 1) / tcells;
