@@ -555,6 +555,19 @@ template <int G>
 __global__ void __launch_bounds__(128) line_fp_queue_kernel(const Launch L) {
   persistent_loop(L, [&](int unit) { line_fp_body<G, false>(L, unit); });
 }
+// Scans alone, pairs and larger groups in one launch, whose CTAs fill each
+// other's last waves (a batch of seven 256^2 slices in a three, a pair and two
+// alone: 160 -> 86 us a forward projection).
+__device__ __forceinline__ void line_fp_any_body(const Launch &L, int unit) {
+  const int nm = L.scans[find_scan(L.prefix, L.nscans, unit)].nmem;
+  if (nm >= 3) line_fp_body<kGroupMax, false>(L, unit);
+  else if (nm == 2) line_fp_body<2, false>(L, unit);
+  else line_fp_body<1, false>(L, unit);
+}
+__global__ void __launch_bounds__(128, 7) line_fp_any_kernel(const Launch L) { line_fp_any_body(L, blockIdx.x); }
+__global__ void __launch_bounds__(128, 7) line_fp_any_queue_kernel(const Launch L) {
+  persistent_loop(L, [&](int unit) { line_fp_any_body(L, unit); });
+}
 
 
 // ---------------------------------------------------------------------------
@@ -1278,9 +1291,10 @@ cudaError_t launch_fp(const Launch &L, int kind, int rpt, int nctas, cudaStream_
 }
 // Forward projection of a batch whose scans sharing a plan are grouped: the
 // members' inputs are interleaved (over the pixel-pass CTAs of Lpix), then
-// each group's rays are walked once, one ray per thread, in one launch per
-// form: groups of three or four over L's CTAs, scans alone over L1's, pairs
-// over L2's.  Returns the number of launches.
+// each group's rays are walked once, one ray per thread: lines in one launch
+// over L's CTAs, by slabs or decision bits in one per form, groups of three or
+// four over L's CTAs, scans alone over L1's, pairs over L2's.  Returns the
+// number of launches.
 int launch_fp_group(const Launch &L, const Launch &Lpix, const Launch &L1, const Launch &L2, int nctas, int pix_nctas,
                     int nctas1, int nctas2, const SlabLaunch *slab, cudaStream_t st) {
   int n = 1;
@@ -1300,11 +1314,15 @@ int launch_fp_group(const Launch &L, const Launch &Lpix, const Launch &L1, const
   Launch Lg = L, Lg1 = L1, Lg2 = L2;
   Lg.tr = Lg1.tr = Lg2.tr = 1;
   if (L.forms & 2) {
-    static int res4 = 0, res1 = 0, res2 = 0;
-    launch_maybe_queued(line_fp_kernel<kGroupMax>, line_fp_queue_kernel<kGroupMax>, res4, Lg, nctas, kFpGroupThreads,
-                        st);
-    launch_maybe_queued(line_fp_kernel<1>, line_fp_queue_kernel<1>, res1, Lg1, nctas1, kFpGroupThreads, st);
-    launch_maybe_queued(line_fp_kernel<2>, line_fp_queue_kernel<2>, res2, Lg2, nctas2, kFpGroupThreads, st);
+    static int res4 = 0, res2 = 0, res = 0;
+    n++;
+    if (L.line_forms == 4)
+      launch_maybe_queued(line_fp_kernel<kGroupMax>, line_fp_queue_kernel<kGroupMax>, res4, Lg, nctas,
+                          kFpGroupThreads, st);
+    else if (L.line_forms == 2)
+      launch_maybe_queued(line_fp_kernel<2>, line_fp_queue_kernel<2>, res2, Lg, nctas, kFpGroupThreads, st);
+    else
+      launch_maybe_queued(line_fp_any_kernel, line_fp_any_queue_kernel, res, Lg, nctas, kFpGroupThreads, st);
   }
   if (L.forms & 1) {
     static int res4 = 0, res1 = 0, res2 = 0;
@@ -1312,8 +1330,9 @@ int launch_fp_group(const Launch &L, const Launch &Lpix, const Launch &L1, const
                         kFpGroupThreads, st);
     launch_maybe_queued(fan_fp_kernel<1, 1>, fan_fp_queue_kernel<1, 1>, res1, Lg1, nctas1, kFpGroupThreads, st);
     launch_maybe_queued(fan_fp_kernel<1, 2>, fan_fp_queue_kernel<1, 2>, res2, Lg2, nctas2, kFpGroupThreads, st);
+    n += (nctas > 0) + (nctas1 > 0) + (nctas2 > 0);
   }
-  return n + ((nctas > 0) + (nctas1 > 0) + (nctas2 > 0)) * (L.forms == 3 ? 2 : 1);
+  return n;
 }
 
 // The row-major and transposed copies of an n x n image that the forward

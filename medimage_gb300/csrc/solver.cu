@@ -285,9 +285,10 @@ int Batch::set(const ScanDev *scans, int n, int kind_, int rpt_, cudaStream_t st
     AT_CUDA_TRY(cudaMemcpyAsync(tmaps_d, maps.data(), sizeof(CUtensorMap) * n, cudaMemcpyHostToDevice, st));
   }
   scans = sc.data();
-  forms = bp_forms = 0;
+  forms = bp_forms = line_forms = 0;
   for (const auto &S : sc) {
     forms |= S.line ? 2 : 1;
+    if (S.nmem && S.line) line_forms |= S.nmem >= 3 ? 4 : S.nmem;
     if (S.nmem) bp_forms |= (S.strip ? 8 : 1) << (S.nmem >= 3 ? 2 : S.nmem - 1);
   }
   cone_chunks = 1;
@@ -302,9 +303,10 @@ int Batch::set(const ScanDev *scans, int n, int kind_, int rpt_, cudaStream_t st
       // and the rest (pairs, scans alone) in launches of their own
       const bool big = nm >= 3, small = nm == 1 || nm == 2;
       const int fpc = slab ? slab_ctas(scans[s]) : fp_group_ctas(scans[s]);
-      add(FAM_FP, s, big ? fpc : 0);
-      add(FAM_FP1, s, nm == 1 ? fpc : 0);
-      add(FAM_FP2, s, nm == 2 ? fpc : 0);
+      const bool line = scans[s].line && !slab;  // one launch for all
+      add(FAM_FP, s, big || (small && line) ? fpc : 0);
+      add(FAM_FP1, s, nm == 1 && !line ? fpc : 0);
+      add(FAM_FP2, s, nm == 2 && !line ? fpc : 0);
       const bool strip = scans[s].strip != 0;  // one launch for all
       add(FAM_BP, s, big || (small && strip) ? bp_ctas(scans[s]) : 0);
       add(FAM_BPS, s, small && !strip ? bp_ctas(scans[s]) : 0);
@@ -401,6 +403,7 @@ Launch Batch::base_launch(int family) const {
   L.chunks = cone_chunks;
   L.forms = forms;
   L.bp_forms = bp_forms;
+  L.line_forms = line_forms;
   const bool fp = family == FAM_FP || family == FAM_FP1 || family == FAM_FP2;
   if (persistent && (family == FAM_BP || family == FAM_BPS || (fp && !slab))) {
     L.queue = queue_d;

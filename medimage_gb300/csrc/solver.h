@@ -39,6 +39,7 @@ struct Batch {
   int group = 1;            // largest group of scans sharing a plan (projected together)
   int forms = 0;            // Launch::forms
   int bp_forms = 0;         // Launch::bp_forms
+  int line_forms = 0;       // Launch::line_forms
   int cone_chunks = 1;      // cone beam: chunks of views of the batch's largest back projection
   // fan back projection: Launch::bp_table of the main launch (groups of three
   // or four, or every scan when nothing is grouped) and of the launch of pairs

@@ -168,6 +168,7 @@ struct Launch {
   int group;                     // projector launches: largest group of scans sharing a plan
   int tr;                        // forward projection: the scans' pack buffers hold transposed inputs
   int forms;                     // fan projectors (host side): 1 some scans walk bits, 2 some walk lines
+  int line_forms;                // (host side) groups walked as lines: 1 scans alone, 2 pairs, 4 larger ones
   int bp_forms;                  // fan back projection (host side): bits 0..2 some scans alone / pairs / larger
                                  // groups walk tile runs or gather from the table, bits 3..5 some walk strips
   int bp_table;                  // fan back projection: 0 walk tile runs, 1 gather from pixel tables,
