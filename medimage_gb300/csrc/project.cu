@@ -25,6 +25,7 @@
 #include <type_traits>
 
 #include "epilogue.cuh"
+#include "launch.h"
 #include "line.cuh"
 #include "solver.h"
 
@@ -112,6 +113,7 @@ __device__ __forceinline__ void pack_image_tiles(const float *const (&src)[kGrou
 // forward projection, sinograms (bins = 1, over the sinogram-pass CTAs) before
 // a grouped back projection.
 __global__ void __launch_bounds__(256) fp_pack_kernel(const Launch L, int bins) {
+  chain_begin();
   const int scan = find_scan(L.prefix, L.nscans, blockIdx.x);
   const ScanDev &S = L.scans[scan];
   if (S.nmem == 0 || (S.nmem == 1 && bins)) return;  // a scan alone: its sinogram is read in place
@@ -548,6 +550,7 @@ __device__ __forceinline__ void line_fp_body(const Launch &L, const int unit) {
 
 template <int G>
 __global__ void __launch_bounds__(128) line_fp_kernel(const Launch L) {
+  chain_begin();
   line_fp_body<G, false>(L, blockIdx.x);
 }
 __global__ void __launch_bounds__(512) line_fp_direct_kernel(const Launch L) { line_fp_body<1, true>(L, blockIdx.x); }
@@ -564,7 +567,10 @@ __device__ __forceinline__ void line_fp_any_body(const Launch &L, int unit) {
   else if (nm == 2) line_fp_body<2, false>(L, unit);
   else line_fp_body<1, false>(L, unit);
 }
-__global__ void __launch_bounds__(128, 7) line_fp_any_kernel(const Launch L) { line_fp_any_body(L, blockIdx.x); }
+__global__ void __launch_bounds__(128, 7) line_fp_any_kernel(const Launch L) {
+  chain_begin();
+  line_fp_any_body(L, blockIdx.x);
+}
 __global__ void __launch_bounds__(128, 7) line_fp_any_queue_kernel(const Launch L) {
   persistent_loop(L, [&](int unit) { line_fp_any_body(L, unit); });
 }
@@ -607,11 +613,11 @@ constexpr int bp_copy_stride() {
 
 // max |r| of each scan's input sinogram, in kBpMaxParts partial maxima
 __global__ void __launch_bounds__(256) sino_absmax_kernel(const Launch L) {
-  asm volatile("griddepcontrol.launch_dependents;");  // strip_bp_kernel prepares meanwhile
+  const int zero = chain_begin();  // (strip_bp_kernel prepares meanwhile)
   const int scan = blockIdx.x / kBpMaxParts, part = blockIdx.x % kBpMaxParts;
   const ScanDev &S = scan_of(L, L.scans ? scan : 0);
   if (!flow_active(S, L.flow)) return;
-  const float *__restrict__ sino = S.buf[L.in_buf];
+  const float *__restrict__ sino = S.buf[L.in_buf] + zero;
   float m = 0.f;
   const int step = kBpMaxParts * blockDim.x;
   int i = part * blockDim.x + threadIdx.x;
@@ -1185,7 +1191,8 @@ int resident_ctas(K kernel, int threads) {
 
 // launches `kernel`, or its queue form `qkernel` over the resident CTAs when
 // the launch carries a work queue
-template <typename K>
+// (kDependent: a kernel that begins with chain_begin)
+template <bool kDependent = false, typename K>
 void launch_maybe_queued(K kernel, K qkernel, int &resident, const Launch &L, int nctas, int threads,
                          cudaStream_t st) {
   if (nctas <= 0) return;
@@ -1193,7 +1200,8 @@ void launch_maybe_queued(K kernel, K qkernel, int &resident, const Launch &L, in
     if (resident <= 0) resident = resident_ctas(qkernel, threads);
     qkernel<<<std::min(nctas, resident), threads, 0, st>>>(L);
   } else {
-    kernel<<<nctas, threads, 0, st>>>(L);
+    if (kDependent) launch_dependent(kernel, nctas, threads, 0, st, L);
+    else kernel<<<nctas, threads, 0, st>>>(L);
   }
 }
 
@@ -1255,7 +1263,7 @@ int launch_fp_walk(const Launch &L, int rpt, int nctas, cudaStream_t st) {
   const int forms = launch_forms(L);
   if (forms & 2) {
     static int res = 0;
-    launch_maybe_queued(line_fp_kernel<1>, line_fp_queue_kernel<1>, res, L, nctas, 128, st);
+    launch_maybe_queued<true>(line_fp_kernel<1>, line_fp_queue_kernel<1>, res, L, nctas, 128, st);
   }
   if (!(forms & 1)) return 1;
   if (rpt == 4) {
@@ -1298,7 +1306,7 @@ cudaError_t launch_fp(const Launch &L, int kind, int rpt, int nctas, cudaStream_
 int launch_fp_group(const Launch &L, const Launch &Lpix, const Launch &L1, const Launch &L2, int nctas, int pix_nctas,
                     int nctas1, int nctas2, const SlabLaunch *slab, cudaStream_t st) {
   int n = 1;
-  fp_pack_kernel<<<pix_nctas, 256, 0, st>>>(Lpix, 0);
+  launch_dependent(fp_pack_kernel, pix_nctas, 256, 0, st, Lpix, 0);
   if (slab) {  // every plan of the batch has slab tables of one CTA shape
     const int G[3] = {kGroupMax, 1, 2};
     const Launch *Ls[3] = {&L, &L1, &L2};
@@ -1317,12 +1325,12 @@ int launch_fp_group(const Launch &L, const Launch &Lpix, const Launch &L1, const
     static int res4 = 0, res2 = 0, res = 0;
     n++;
     if (L.line_forms == 4)
-      launch_maybe_queued(line_fp_kernel<kGroupMax>, line_fp_queue_kernel<kGroupMax>, res4, Lg, nctas,
+      launch_maybe_queued<true>(line_fp_kernel<kGroupMax>, line_fp_queue_kernel<kGroupMax>, res4, Lg, nctas,
                           kFpGroupThreads, st);
     else if (L.line_forms == 2)
-      launch_maybe_queued(line_fp_kernel<2>, line_fp_queue_kernel<2>, res2, Lg, nctas, kFpGroupThreads, st);
+      launch_maybe_queued<true>(line_fp_kernel<2>, line_fp_queue_kernel<2>, res2, Lg, nctas, kFpGroupThreads, st);
     else
-      launch_maybe_queued(line_fp_any_kernel, line_fp_any_queue_kernel, res, Lg, nctas, kFpGroupThreads, st);
+      launch_maybe_queued<true>(line_fp_any_kernel, line_fp_any_queue_kernel, res, Lg, nctas, kFpGroupThreads, st);
   }
   if (L.forms & 1) {
     static int res4 = 0, res1 = 0, res2 = 0;
@@ -1340,6 +1348,7 @@ int launch_fp_group(const Launch &L, const Launch &Lpix, const Launch &L1, const
 // tiles (coalesced reads and writes)
 __global__ void __launch_bounds__(256) pack_single_kernel(const float *__restrict__ in, float *__restrict__ out,
                                                            int n, int pitch, int pad) {
+  in += chain_begin();
   __shared__ float t[32][33];
   const int bx = blockIdx.x * 32, by = blockIdx.y * 32;
   float *outt = out + (size_t)n * pitch;
@@ -1377,8 +1386,9 @@ cudaError_t launch_fp_single(const Launch &L, const Plan &p, int rpt, void *scra
   const ScanDev &S = L.single;
   const int n = S.n;
   float *copies = reinterpret_cast<float *>(scratch);
-  pack_single_kernel<<<dim3((n + 31) / 32, (n + 31) / 32), dim3(32, 8), 0, st>>>(S.buf[L.in_buf], copies, n, S.lpitch,
-                                                                                 S.lpad);
+  cudaError_t e = launch_dependent(pack_single_kernel, dim3((n + 31) / 32, (n + 31) / 32), dim3(32, 8), 0, st,
+                                   S.buf[L.in_buf], copies, n, S.lpitch, S.lpad);
+  if (e != cudaSuccess) return e;
   Launch Lt = L;
   Lt.single.pack = reinterpret_cast<float4 *>(copies);
   if (p.slab.ok) {
@@ -1388,7 +1398,7 @@ cudaError_t launch_fp_single(const Launch &L, const Plan &p, int rpt, void *scra
     // (a descriptor the driver refuses reads as "not supported", a launch
     // configuration it refuses as "invalid argument")
     if (encode_pack_tmap(&hmap, copies, n, S.lpitch, 1, p.slab.wbox, p.slab.rows)) return cudaErrorNotSupported;
-    cudaError_t e = cudaMemcpyAsync(dmap, &hmap, sizeof(hmap), cudaMemcpyHostToDevice, st);
+    e = cudaMemcpyAsync(dmap, &hmap, sizeof(hmap), cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return e;
     Lt.single.tmap = dmap;
     return launch_fp_slab(Lt, 1, p.slab.ncta, p.slab.views * p.slab.rays,
@@ -1407,7 +1417,7 @@ cudaError_t launch_fp_single(const Launch &L, const Plan &p, int rpt, void *scra
 // Returns the number of launches.
 int launch_fp_tr(const Launch &L, const Launch &Lpix, int rpt, int nctas, int pix_nctas, const SlabLaunch *slab,
                  cudaStream_t st) {
-  fp_pack_kernel<<<pix_nctas, 256, 0, st>>>(Lpix, 0);
+  launch_dependent(fp_pack_kernel, pix_nctas, 256, 0, st, Lpix, 0);
   if (slab) {
     const int nl = launch_fp_slab(L, 1, nctas, slab->threads, slab->smem[1], st);
     return nl < 0 ? -1 : 1 + nl;
@@ -1430,8 +1440,8 @@ int launch_bp_group(const Launch &L, const Launch &Lsino, const Launch &Lsmall, 
   int n = 2;
   Launch La = L;  // the max |r| pass: one CTA per part, never queued
   La.queue = nullptr;
-  sino_absmax_kernel<<<L.nscans * kBpMaxParts, 256, 0, st>>>(La);
-  fp_pack_kernel<<<sino_nctas, 256, 0, st>>>(Lsino, 1);
+  launch_dependent(sino_absmax_kernel, L.nscans * kBpMaxParts, 256, 0, st, La);
+  launch_dependent(fp_pack_kernel, sino_nctas, 256, 0, st, Lsino, 1);
   static int resg[3] = {0, 0, 0}, ress[3] = {0, 0, 0};
   auto group = [&](auto kern, int m) {
     launch_maybe_queued(kern, fan_bp_group_queue_kernel, resg[m], L, nctas, 256, st);
@@ -1470,7 +1480,7 @@ cudaError_t launch_bp(const Launch &L, int kind, int nctas, cudaStream_t st, con
     La.queue = nullptr;
     const int forms = L.scans ? L.bp_forms : L.single.strip ? 8 : 1;
     La.flag = !L.scans && forms == 8;
-    sino_absmax_kernel<<<(L.scans ? L.nscans : 1) * kBpMaxParts, 256, 0, st>>>(La);
+    launch_dependent(sino_absmax_kernel, (L.scans ? L.nscans : 1) * kBpMaxParts, 256, 0, st, La);
     if (forms & 56) {
       if (!Lpix) return cudaErrorInvalidValue;
       cudaError_t e = launch_strip_bp(L, nctas, st);

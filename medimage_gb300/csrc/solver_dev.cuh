@@ -218,6 +218,22 @@ struct SlabLaunch {
   size_t smem[3];
 };
 
+// The kernels of a projection follow each other with programmatic
+// serialisation (launch.h): a kernel's CTAs may be on the SMs before the kernel
+// before it has ended, and wait here for its end (and, each kernel waiting so,
+// for that of all before it) ahead of their first load of what those wrote.
+// One projection of 64^2 14.2 -> 11.6 us, one back projection of 217^2 46 -> 35
+// us.  (The passes between projections gain nothing in a solver's graph.)
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// ... and lets the next kernel's CTAs come as soon as all of this one's have.
+// Returns 0, for a first load whose address is a kernel parameter's: added to
+// it, the load cannot be moved ahead of the wait.
+__device__ __forceinline__ int chain_begin() {
+  int zero;
+  asm volatile("griddepcontrol.wait;\ngriddepcontrol.launch_dependents;\nmov.b32 %0, 0;" : "=r"(zero) : : "memory");
+  return zero;
+}
+
 __device__ __forceinline__ int find_scan(const int *prefix, int nscans, int cta) {
   int lo = 0, hi = nscans;  // prefix[lo] <= cta < prefix[hi]
   while (hi - lo > 1) {

@@ -35,6 +35,7 @@
 #include <vector>
 
 #include "epilogue.cuh"
+#include "launch.h"
 #include "line.cuh"
 #include "solver.h"
 
@@ -83,11 +84,6 @@ __host__ __device__ inline int strip_cells_of(int n, int ncc) {
   const int tc = strip_tile_cells(ncc, StripShape<G>::cols);
   return ((n + StripShape<G>::rows - 1) / StripShape<G>::rows) * ((ncc + tc - 1) / tc);
 }
-
-// Launches after the kernel before them with programmatic serialisation (the
-// chain of three short kernels of a small back projection would else wait for
-// each other's launches): what they read of it comes after this.
-__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 __device__ __forceinline__ void red_global_add(unsigned long long *p, int v) {
   asm volatile("red.global.add.u64 [%0], %1;" ::"l"(p), "l"((long long)v) : "memory");
@@ -380,7 +376,7 @@ __global__ void __launch_bounds__(kStripThreads, 3) strip_bp_kernel(const Launch
 // The sums as pixels, through the solver's epilogue; leaves zeros.  Over the
 // pixel-pass CTAs.
 __global__ void __launch_bounds__(256) strip_finish_kernel(const Launch L) {
-  grid_dependency_wait();
+  chain_begin();
   const int scan = L.scans ? find_scan(L.prefix, L.nscans, blockIdx.x) : 0;
   const ScanDev &S = scan_of(L, scan);
   if (!S.strip || !flow_active(S, L.flow)) return;
@@ -427,21 +423,6 @@ int strip_cells(const ScanDev &S, int nmem) {
 }
 }  // namespace
 
-template <typename K>
-cudaError_t launch_dependent(K kernel, const Launch &L, int nctas, int threads, size_t smem, cudaStream_t st) {
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(nctas);
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, L);
-}
-
 cudaError_t launch_strip_bp(const Launch &L, int nctas, cudaStream_t st) {
   static std::once_flag once;
   static cudaError_t err = cudaSuccess;
@@ -449,11 +430,11 @@ cudaError_t launch_strip_bp(const Launch &L, int nctas, cudaStream_t st) {
     err = cudaFuncSetAttribute(strip_bp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStripSmem);
   });
   if (err != cudaSuccess) return err;
-  return launch_dependent(strip_bp_kernel, L, nctas, kStripThreads, kStripSmem, st);
+  return launch_dependent(strip_bp_kernel, nctas, kStripThreads, kStripSmem, st, L);
 }
 
 cudaError_t launch_strip_finish(const Launch &Lpix, int pix_nctas, cudaStream_t st) {
-  return launch_dependent(strip_finish_kernel, Lpix, pix_nctas, 256, 0, st);
+  return launch_dependent(strip_finish_kernel, pix_nctas, 256, 0, st, Lpix);
 }
 
 // CTAs of a scan (or the group it leads)
