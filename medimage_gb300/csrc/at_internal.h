@@ -125,7 +125,22 @@ constexpr unsigned kSlabDown = 2u;        // its rays run towards decreasing row
 constexpr unsigned kSlabFallback = 4u;    // a ray leaves the grid or runs against the others: gather through L1
 constexpr unsigned kSlabEmpty = 8u;       // no ray of the CTA crosses the image
 
+// Stream-ordered scratch of single calls, from a pool of the library's own that
+// keeps up to kScratchKept bytes between calls: the driver's default pool hands
+// everything back whenever the host waits for the GPU, and each call after a
+// wait then maps its scratch anew (190 us at any size).  The last plan to go
+// gives all of it back.  Freed with cudaFreeAsync.
+constexpr uint64_t kScratchKept = 512ull << 20;
+cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t st);
+struct ScratchUser {
+  ScratchUser();
+  ~ScratchUser();
+  ScratchUser(const ScratchUser &) = delete;
+  ScratchUser &operator=(const ScratchUser &) = delete;
+};
+
 struct Plan {
+  ScratchUser scratch_user;
   int kind = AT_GEOM_FAN;
   at_fan_geometry geom{};
   int n = 0, nviews = 0, ndets = 0;

@@ -41,6 +41,60 @@ int cuda_error(cudaError_t e, const char *what) {
   return set_error(code, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
+// ------------------------------------------------------------ scratch pools
+namespace {
+constexpr int kMaxDevices = 64;
+struct ScratchPools {
+  std::mutex mu;
+  cudaMemPool_t pool[kMaxDevices] = {};
+  int plans = 0;
+};
+// (never destroyed: plans may outlive static objects)
+ScratchPools &scratch_pools() {
+  static ScratchPools *const p = new ScratchPools;
+  return *p;
+}
+}  // namespace
+
+ScratchUser::ScratchUser() {
+  ScratchPools &P = scratch_pools();
+  std::lock_guard<std::mutex> lock(P.mu);
+  P.plans++;
+}
+
+ScratchUser::~ScratchUser() {
+  ScratchPools &P = scratch_pools();
+  std::lock_guard<std::mutex> lock(P.mu);
+  if (--P.plans) return;
+  for (cudaMemPool_t pool : P.pool)  // (what calls in flight hold stays theirs)
+    if (pool) cudaMemPoolTrimTo(pool, 0);
+}
+
+cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t st) {
+  *p = nullptr;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev >= kMaxDevices) return cudaMallocAsync(p, bytes, st);
+  cudaMemPool_t pool;
+  {
+    ScratchPools &P = scratch_pools();
+    std::lock_guard<std::mutex> lock(P.mu);
+    if (!P.pool[dev]) {
+      cudaMemPoolProps props{};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.handleTypes = cudaMemHandleTypeNone;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = dev;
+      if ((e = cudaMemPoolCreate(&P.pool[dev], &props)) != cudaSuccess) return e;
+      uint64_t kept = kScratchKept;
+      if ((e = cudaMemPoolSetAttribute(P.pool[dev], cudaMemPoolAttrReleaseThreshold, &kept)) != cudaSuccess) return e;
+    }
+    pool = P.pool[dev];
+  }
+  return cudaMallocFromPoolAsync(p, bytes, pool, st);
+}
+
 namespace {
 
 int projector_rpt(const Plan &p) {
@@ -68,7 +122,7 @@ int project(const Plan &p, bool forward, const float *in, float *out, cudaStream
     if (p.kind == AT_GEOM_FAN || p.kind == AT_GEOM_RAYS) {
       // stream-ordered scratch for the image's row-major and transposed copies
       void *tr = nullptr;
-      AT_CUDA_TRY(cudaMallocAsync(&tr, fp_single_scratch_bytes(p), st));
+      AT_CUDA_TRY(scratch_alloc(&tr, fp_single_scratch_bytes(p), st));
       e = launch_fp_single(L, p, rpt, tr, st);
       cudaFreeAsync(tr, st);
     } else {
@@ -79,7 +133,7 @@ int project(const Plan &p, bool forward, const float *in, float *out, cudaStream
     const size_t bpb = bp_scratch_bytes(p);
     void *scratch = nullptr;
     if (bpb) {
-      AT_CUDA_TRY(cudaMallocAsync(&scratch, bpb, st));
+      AT_CUDA_TRY(scratch_alloc(&scratch, bpb, st));
       // (scratch that strips use is cleared by their first kernel)
       if (!L.single.strip && (e = cudaMemsetAsync(scratch, 0, bpb, st)) != cudaSuccess) {
         cudaFreeAsync(scratch, st);
@@ -366,7 +420,8 @@ int project_host(const Plan &p, bool forward, const float *h_in, float *h_out) {
   int rc = AT_OK;
   cudaError_t e;
   if ((e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking)) != cudaSuccess) return cuda_error(e, "stream");
-  if ((e = cudaMallocAsync(&din, nin * 4, st)) != cudaSuccess || (e = cudaMallocAsync(&dout, nout * 4, st)) != cudaSuccess) {
+  if ((e = scratch_alloc((void **)&din, nin * 4, st)) != cudaSuccess ||
+      (e = scratch_alloc((void **)&dout, nout * 4, st)) != cudaSuccess) {
     rc = cuda_error(e, "cudaMallocAsync");
   } else if ((e = cudaMemcpyAsync(din, h_in, nin * 4, cudaMemcpyHostToDevice, st)) != cudaSuccess) {
     rc = cuda_error(e, "H2D");
