@@ -117,15 +117,12 @@ __global__ void __launch_bounds__(256) fp_pack_kernel(const Launch L, int bins) 
   const int scan = find_scan(L.prefix, L.nscans, blockIdx.x);
   const ScanDev &S = L.scans[scan];
   if (S.nmem == 0 || (S.nmem == 1 && bins)) return;  // a scan alone: its sinogram is read in place
+  const unsigned act = group_active<kGroupMax>(L, S);
+  if (!act) return;
   const float *src[kGroupMax];
-  bool any = false;
 #pragma unroll
-  for (int m = 0; m < kGroupMax; m++) {
-    const ScanDev &Mm = L.scans[S.mem[m < S.nmem ? m : 0]];
-    src[m] = (m < S.nmem && flow_active(Mm, L.flow)) ? Mm.buf[L.in_buf] : nullptr;
-    any |= src[m] != nullptr;
-  }
-  if (!any) return;
+  for (int m = 0; m < kGroupMax; m++)
+    src[m] = ((act >> m) & 1u) ? L.scans[S.mem[m]].buf[L.in_buf] : nullptr;
   const int cta0 = __ldg(L.prefix + scan), ncta = __ldg(L.prefix + scan + 1) - cta0;
   const int local = blockIdx.x - cta0;
   if (!bins) {

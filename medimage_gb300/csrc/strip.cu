@@ -16,8 +16,8 @@
 // stream (288 MB at 512^2, 720 x 888), no decision bits, and the lanes of a
 // warp, neighbouring rays in the same row, add side by side instead of in a
 // dozen rows of a small tile (two wavefronts an add for almost four).  512^2,
-// 720 x 888: one slice 287 -> 184 us, sixteen slices 2.51 -> 1.84 ms; 1024^2,
-// 1440 x 1536: 1.70 -> 1.00 ms; error against 64 bits 5.9e-7 -> 2e-7 (a
+// 720 x 888: one slice 287 -> 182 us, sixteen slices 2.51 -> 1.74 ms; 1024^2,
+// 1440 x 1536: 1.70 -> 1.03 ms; error against 64 bits 5.9e-7 -> 2e-7 (a
 // crossing is rounded as a row number, not as a distance from the source).
 // Bound: the L1 data pipe (88 % of its wavefronts while CTAs run; two an add,
 // because 32 neighbouring rays cover either more or fewer than 32 columns).
@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(256) strip_finish_kernel(const Launch L) {
   float mx = fmaxf(S.bpmax[lane], S.bpmax[lane + 32]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  const double unit = ldexp(1.0, -strip_scale_exp(S, mx));
+  const float unit = ldexpf(1.f, -strip_scale_exp(S, mx));  // (a power of two: one rounding, the conversion's)
   const int y = (local % nt) * 32 + lane, x0 = (local / nt) * kPixRows + warp;
   constexpr int kRowsEach = kPixRows / 8;
   long long t[kRowsEach];
@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(256) strip_finish_kernel(const Launch L) {
     const int x = x0 + r * 8;
     if (x >= n || y >= n) continue;
     if (t[r]) S.bp_acc[x * n + y] = 0ull;
-    bp_epilogue(S, L, 0, x, y, (float)((double)t[r] * unit), s0[0]);
+    bp_epilogue(S, L, 0, x, y, __ll2float_rn(t[r]) * unit, s0[0]);
   }
   if (stage_reduces(L.stage)) reduce_and_finalize<1>(S, L, s0, local, ncta);
 }
@@ -442,15 +442,15 @@ int strip_ctas(const ScanDev &S) { return S.strip_npart * strip_cells(S, std::ma
 
 // Chooses the division of the views for a launch, by an estimate of the items
 // (32 rays through a strip) that the busiest SM goes through: its CTAs' items
-// and, for each CTA, the 12 that its own passes over its sums are worth.  Up to
-// three CTAs on every SM run at once: the strips' differences stay (1.35), and
+// and, for each CTA, the 30 that its own passes over its sums are worth.  Up to
+// three CTAs on every SM run at once: the strips' differences stay (1.75), and
 // an SM with fewer of them waits more.  Beyond, CTAs follow as others end, and
-// the last ones leave SMs idle for 1.5 of them.  Fitted to sweeps over the
+// the last ones leave SMs idle for three of them.  Fitted to sweeps over the
 // divisions (one slice of 217^2: 392 CTAs 44 us, 672 48 us; 512^2: 448 CTAs 198
-// us, 1536 187 us; sixteen slices of 512^2: 6144 CTAs 1.82 ms, 14336 1.97 ms).
-// Results do not depend on it.
+// us, 1536 187 us; 1024^2: 2944 CTAs 1.08 ms, 6144 1.00 ms; sixteen slices of
+// 512^2: 6144 CTAs 1.82 ms, 14336 1.97 ms).  Results do not depend on it.
 void strip_choose(ScanDev *scans, int n) {
-  constexpr double kOwn = 12.0, kSms = 152.0;
+  constexpr double kOwn = 30.0, kSms = 152.0;
   auto set = [&](int q) {
     for (int s = 0; s < n; s++) {
       if (!scans[s].strip) continue;
@@ -471,8 +471,8 @@ void strip_choose(ScanDev *scans, int n) {
     }
     if (ctas == 0.0) return;
     const double per = std::ceil(ctas / kSms);
-    const double t = per <= 3.0 ? per * (1.35 * items / ctas + kOwn) / (per == 1.0 ? 0.6 : per == 2.0 ? 0.85 : 1.0)
-                                : (ctas / kSms + 1.5) * (items / ctas + kOwn);
+    const double t = per <= 3.0 ? per * (1.75 * items / ctas + kOwn) / (per == 1.0 ? 0.55 : per == 2.0 ? 0.85 : 1.0)
+                                : (ctas / kSms + 3.0) * (items / ctas + kOwn);
     if (t < best) {
       best = t;
       pick = q;
