@@ -442,15 +442,16 @@ int strip_ctas(const ScanDev &S) { return S.strip_npart * strip_cells(S, std::ma
 
 // Chooses the division of the views for a launch, by an estimate of the items
 // (32 rays through a strip) that the busiest SM goes through: its CTAs' items
-// and, for each CTA, the 30 that its own passes over its sums are worth.  Up to
-// three CTAs on every SM run at once: the strips' differences stay (1.75), and
-// an SM with fewer of them waits more.  Beyond, CTAs follow as others end, and
-// the last ones leave SMs idle for three of them.  Fitted to sweeps over the
-// divisions (one slice of 217^2: 392 CTAs 44 us, 672 48 us; 512^2: 448 CTAs 198
+// and what each CTA's own passes over its sums are worth.  Up to three CTAs on
+// every SM run at once: their own passes overlap (12 items), the strips'
+// differences stay (1.75), and an SM with fewer of them waits more.  Beyond,
+// CTAs follow as others end (30 items), and the last ones leave SMs idle for
+// three of them.  Fitted to sweeps over the divisions (one slice of 100^2: 144
+// CTAs 18 us, 288 16 us; 217^2: 392 CTAs 34 us, 672 38 us; 512^2: 448 CTAs 198
 // us, 1536 187 us; 1024^2: 2944 CTAs 1.08 ms, 6144 1.00 ms; sixteen slices of
 // 512^2: 6144 CTAs 1.82 ms, 14336 1.97 ms).  Results do not depend on it.
 void strip_choose(ScanDev *scans, int n) {
-  constexpr double kOwn = 30.0, kSms = 152.0;
+  constexpr double kOwn = 30.0, kOwnBeside = 12.0, kSms = 152.0;
   auto set = [&](int q) {
     for (int s = 0; s < n; s++) {
       if (!scans[s].strip) continue;
@@ -471,7 +472,7 @@ void strip_choose(ScanDev *scans, int n) {
     }
     if (ctas == 0.0) return;
     const double per = std::ceil(ctas / kSms);
-    const double t = per <= 3.0 ? per * (1.75 * items / ctas + kOwn) / (per == 1.0 ? 0.55 : per == 2.0 ? 0.85 : 1.0)
+    const double t = per <= 3.0 ? per * (1.75 * items / ctas + kOwnBeside) / (per == 1.0 ? 0.55 : per == 2.0 ? 0.75 : 1.0)
                                 : (ctas / kSms + 3.0) * (items / ctas + kOwn);
     if (t < best) {
       best = t;
