@@ -16,8 +16,8 @@
 // stream (288 MB at 512^2, 720 x 888), no decision bits, and the lanes of a
 // warp, neighbouring rays in the same row, add side by side instead of in a
 // dozen rows of a small tile (two wavefronts an add for almost four).  512^2,
-// 720 x 888: one slice 287 -> 182 us, sixteen slices 2.51 -> 1.74 ms; 1024^2,
-// 1440 x 1536: 1.70 -> 1.03 ms; error against 64 bits 5.9e-7 -> 2e-7 (a
+// 720 x 888: one slice 287 -> 180 us, sixteen slices 2.51 -> 1.72 ms; 1024^2,
+// 1440 x 1536: 1.70 -> 1.02 ms; error against 64 bits 5.9e-7 -> 2e-7 (a
 // crossing is rounded as a row number, not as a distance from the source).
 // Bound: the L1 data pipe (88 % of its wavefronts while CTAs run; two an add,
 // because 32 neighbouring rays cover either more or fewer than 32 columns).
