@@ -452,11 +452,29 @@ int strip_ctas(const ScanDev &S) { return S.strip_npart * strip_cells(S, std::ma
 // 512^2: 6144 CTAs 1.82 ms, 14336 1.97 ms).  Results do not depend on it.
 void strip_choose(ScanDev *scans, int n) {
   constexpr double kOwn = 30.0, kOwnBeside = 12.0, kSms = 152.0;
+  auto items_of = [](const ScanDev &S) { return (double)S.nbins / 32.0 * strip_cells(S, std::max(1, S.nmem)) / 1.5; };
+  auto take = [](ScanDev &S, int q) {
+    S.strip_parts = S.strip_part0 + S.strip_poff[q];
+    S.strip_npart = S.strip_poff[q + 1] - S.strip_poff[q];
+  };
+  int most = -1;  // the scan with the most work
+  for (int s = 0; s < n; s++)
+    if (scans[s].strip && scans[s].nmem && (most < 0 || items_of(scans[s]) > items_of(scans[most]))) most = s;
+  bool groups = false;
+  for (int s = 0; s < n; s++) groups |= scans[s].nmem > 1;
+  // division q for that scan, and for the others the coarsest whose CTAs have
+  // no more work than its (scans of 241^2 and 160^2: 56 -> 47 us); with groups,
+  // whose items cost more than a single scan's, q for all (302^2, a pair and
+  // one alone: 111 us against 202)
   auto set = [&](int q) {
+    if (most >= 0) take(scans[most], q);
+    const double each = most < 0 ? 0.0 : items_of(scans[most]) / strip_ctas(scans[most]);
     for (int s = 0; s < n; s++) {
-      if (!scans[s].strip) continue;
-      scans[s].strip_parts = scans[s].strip_part0 + scans[s].strip_poff[q];
-      scans[s].strip_npart = scans[s].strip_poff[q + 1] - scans[s].strip_poff[q];
+      if (!scans[s].strip || s == most) continue;
+      for (int p = groups ? q : 0; p <= q; p++) {
+        take(scans[s], p);
+        if (items_of(scans[s]) / strip_ctas(scans[s]) <= 1.15 * each) break;
+      }
     }
   };
   double best = 1e300;
@@ -468,7 +486,7 @@ void strip_choose(ScanDev *scans, int n) {
       const ScanDev &S = scans[s];
       if (!S.strip || !S.nmem) continue;
       ctas += strip_ctas(S);
-      items += (double)S.nbins / 32.0 * strip_cells(S, S.nmem) / 1.5;
+      items += items_of(S);
     }
     if (ctas == 0.0) return;
     const double per = std::ceil(ctas / kSms);
