@@ -392,6 +392,12 @@ __global__ void max_kernel(const unsigned *v, size_t n, unsigned *out) {
   if ((threadIdx.x & 31) == 0) atomicMax(out, m);
 }
 
+// *out = max(*out, v[0..n-1])
+cudaError_t launch_max(const unsigned *v, size_t n, unsigned *out, cudaStream_t st) {
+  max_kernel<<<256, 256, 0, st>>>(v, n, out);
+  return cudaGetLastError();
+}
+
 namespace {
 template <typename T>
 int dev_alloc(T **p, size_t count, int64_t &acct) {
@@ -567,8 +573,7 @@ int build_fan_runs(Plan &p, cudaStream_t st) {
       pixel_hits_kernel<<<((v1 - v0) * p.ndets + 127) / 128, 128, 0, st>>>(p.n, v0, v1, p.ndets, p.nblocks_per_view,
                                                                           p.rays_d, p.bits_d, p.blk_word_d, hits);
       AT_CUDA_TRY(cudaGetLastError());
-      max_kernel<<<256, 256, 0, st>>>(hits, cells, mx);
-      AT_CUDA_TRY(cudaGetLastError());
+      AT_CUDA_TRY(launch_max(hits, cells, mx, st));
     }
     unsigned m = 0;
     AT_CUDA_TRY(cudaMemcpyAsync(&m, mx, sizeof(m), cudaMemcpyDeviceToHost, st));
@@ -720,8 +725,8 @@ int build_fan_plan(Plan &p, cudaStream_t st, const double *h_ends) {
     fan_fill_kernel<double><<<(nrays + tpb - 1) / tpb, tpb, 0, st>>>(R, p.nblocks_per_view, p.blk_word_d, p.bits_d);
   AT_CUDA_TRY(cudaGetLastError());
 
-  if ((rc = build_lines(p, R, st))) return rc;
   if ((rc = build_fan_runs(p, st))) return rc;
+  if ((rc = build_lines(p, R, st))) return rc;
   AT_CUDA_TRY(cudaStreamSynchronize(st));
   cudaFree(tab_d);
   return AT_OK;

@@ -41,6 +41,8 @@
 
 namespace medimg {
 
+cudaError_t launch_max(const unsigned *v, size_t n, unsigned *out, cudaStream_t st);
+
 namespace {
 
 // Strip of G members' sums.  About 66 KB: three CTAs per SM.
@@ -539,16 +541,83 @@ __global__ void strip_range_kernel(int n, int nviews, int ndets, int ncr, int nc
   if (any) atomicAdd(count + 2 * view + dir, 1u);
 }
 
+// What the strips add to each pixel in the views [view0, view1), in 1/64 of a
+// whole row of a ray (each part rounded up): the same steps as strip_row.
+constexpr unsigned kHitsUnit = 64;
+__global__ void strip_hits_kernel(int n, int view0, int view1, int ndets, int ncr, const LineRay *line,
+                                  unsigned *hits) {
+  const int ray = view0 * ndets + blockIdx.x * blockDim.x + threadIdx.x;
+  if (ray >= view1 * ndets) return;
+  const LineRay r = load_line(line + ray);
+  LineWalk<1> w;
+  w.load(r);
+  if (w.empty()) return;
+  const bool swap = (r.flags & kLineSwap) != 0, down = (r.flags & kLineDown) != 0;
+  const int col0 = line_c0(r, n, line_pitch(n));
+  auto add = [&](int u, int c, float part) {
+    if ((unsigned)u < (unsigned)n && (unsigned)c < (unsigned)n && part > 0.f)
+      atomicAdd(hits + (swap ? (size_t)c * n + u : (size_t)u * n + c), (unsigned)ceilf(part * kHitsUnit));
+  };
+  for (int cr = 0; cr < ncr; cr++) {
+    const int u0 = cr * kStripCellRows;
+    const int step0 = down ? n - u0 - kStripCellRows : u0;
+    if (w.last < step0 || w.first >= step0 + kStripCellRows) continue;
+    int c = col0 + w.enter(step0, n);
+    for (int b = 0; b < kStripCellRows; b++) {
+      const float f = w.before((float)b);
+      const bool x = w.crosses((float)b);
+      const int u = line_row_of(r, step0 + b, n);
+      add(u, c, f);
+      if (x) add(u, ++c, 1.f - f);
+    }
+  }
+}
+
+// Whether the strips' 32-bit sums hold whatever kBpViewBlock views add to a
+// pixel.  A term is at most part * (len / 1.5 pixel) * 2^bp_term_bits, len at
+// most sqrt(2) pixels, and rounded by half a unit, so the parts' sum bounds the
+// terms' in units of 2^bp_term_bits.  Fan beams: the geometric bound that
+// bp_term_bits comes from covers every ray through a pixel.  Ray tables: it
+// counts the segments of the traversal, which leaves out the last 0.05 mm of
+// each ray; the strips add those too (and take them back in 64 bits), so what
+// they add is counted here.
+int strips_fit(const Plan &p, int ncr, cudaStream_t st, bool *fit) {
+  *fit = true;
+  if (p.kind == AT_GEOM_FAN) return AT_OK;
+  const size_t cells = (size_t)p.n * p.n;
+  unsigned *hits = nullptr;
+  const auto free_hits = scope_exit([&] { cudaFree(hits); });
+  AT_CUDA_TRY(cudaMalloc(&hits, sizeof(unsigned) * (cells + 1)));
+  unsigned *const mx = hits + cells;
+  AT_CUDA_TRY(cudaMemsetAsync(mx, 0, sizeof(unsigned), st));
+  for (int v0 = 0; v0 < p.nviews; v0 += kBpViewBlock) {
+    const int v1 = std::min(p.nviews, v0 + kBpViewBlock);
+    AT_CUDA_TRY(cudaMemsetAsync(hits, 0, sizeof(unsigned) * cells, st));
+    strip_hits_kernel<<<((v1 - v0) * p.ndets + 127) / 128, 128, 0, st>>>(p.n, v0, v1, p.ndets, ncr, p.line_d, hits);
+    AT_CUDA_TRY(cudaGetLastError());
+    AT_CUDA_TRY(launch_max(hits, cells, mx, st));
+  }
+  unsigned most = 0;
+  AT_CUDA_TRY(cudaMemcpyAsync(&most, mx, sizeof(most), cudaMemcpyDeviceToHost, st));
+  AT_CUDA_TRY(cudaStreamSynchronize(st));
+  *fit = (uint64_t)most << p.bp_term_bits < (uint64_t)kHitsUnit << 31;
+  return AT_OK;
+}
+
 __global__ void strip_none_kernel(int2 *rng, size_t cells) {
   const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i < cells) rng[i] = make_int2(INT_MAX, -1);
 }
 
-// The tables of the strip back projector.  `off`: first correction of each ray
-// and, at the end, how many there are; `corr` the corrections.
+// The tables of the strip back projector; none where its sums might not fit
+// (bp_term_bits is known by now).  `off`: first correction of each ray and, at
+// the end, how many there are; `corr` the corrections.
 int build_strips(Plan &p, const std::vector<int> &off, const std::vector<LineCorr> &corr, cudaStream_t st) {
   const int n = p.n, nrays = p.nviews * p.ndets;
   const int ncr = (n + kStripCellRows - 1) / kStripCellRows, ncc = (n + kStripCellCols - 1) / kStripCellCols;
+  bool fit;
+  if (const int rc = strips_fit(p, ncr, st, &fit)) return rc;
+  if (!fit) return AT_OK;  // (tile runs keep the scale, and with it the precision)
   const size_t cells = (size_t)p.nviews * 2 * ncr * ncc;
   unsigned *count_d = nullptr;
   const auto free_temps = scope_exit([&] { cudaFree(count_d); });
