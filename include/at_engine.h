@@ -373,7 +373,9 @@ int at_server_get_stats(const at_server *s, at_server_stats *out);
  * computes d_r = d_g - A d_img and *d_energy = sum (A d_img - d_g)^2 (FP64,
  * device pointer) with the forward projector and its fused reduction, taking
  * the reduction's scratch from a fixed 256 KiB array compiled into the
- * library instead of allocating it.  Plans whose forward projection needs more
+ * library instead of allocating it, and writing the copies of the image that
+ * the walk along lines reads into memory that the plan holds for it (counted
+ * in at_plan_stats.device_bytes).  Plans whose forward projection needs more
  * than that (more than about 32,700 CTAs) are rejected with AT_EINVAL.  The
  * first call on a device looks up the array's address (make it before any
  * stream capture); calls share the array, so calls that overlap on the GPU

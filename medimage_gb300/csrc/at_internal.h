@@ -171,6 +171,7 @@ struct Plan {
   LineRay *line_d = nullptr;
   LineCorr *lcorr_d = nullptr;
   int64_t ncorr = 0;
+  float *copies_d = nullptr;  // the image's copies, for the call that allocates nothing
   // back projection along the lines (strip.cu), the default where there are
   // lines: per view, direction (rows along x or y) and cell the first and last
   // detector whose ray meets the cell; the ranges of views a CTA takes,

@@ -620,6 +620,7 @@ int build_lines(Plan &p, const RaySource &R, cudaStream_t st) {
   off[nrays] = (int)tot;
   int rc;
   if ((rc = dev_alloc(&p.lcorr_d, tot, p.device_bytes))) return rc;
+  if ((rc = dev_alloc(&p.copies_d, 2 * (size_t)p.n * line_pitch(p.n), p.device_bytes))) return rc;
   AT_CUDA_TRY(cudaMemcpyAsync(cnt_d, off.data(), sizeof(int) * ((size_t)nrays + 1), cudaMemcpyHostToDevice, st));
   line_corr_kernel<<<(nrays + tpb - 1) / tpb, tpb, 0, st>>>(R, first, cnt_d, line, p.lcorr_d);
   AT_CUDA_TRY(cudaGetLastError());
@@ -959,6 +960,7 @@ Plan::~Plan() {
   cudaFree(blk_off_d);
   cudaFree(line_d);
   cudaFree(lcorr_d);
+  cudaFree(copies_d);
   cudaFree(strip_rng_d);
   cudaFree(strip_part_d);
   cudaFree(strip_corr_d);

@@ -417,12 +417,9 @@ __global__ void __launch_bounds__(128) fan_fp_queue_kernel(const Launch L) {
 // L1 at C2), the L1 data path for four (84 %: 2 x 16 bytes a row and lane).
 // C2, the image's copies included: one slice 243 -> 130 us, eight slices
 // 812 -> 560 us; error against 64 bits 2.2e-7 -> 1.3e-7.
-// kDirect: the image itself instead of the padded copies, every column checked
-// (the call that may not allocate); the same sums.
-template <int G, bool kDirect>
+template <int G>
 __device__ __forceinline__ void line_fp_body(const Launch &L, const int unit) {
   using T = typename Elem<G>::T;
-  static_assert(G == 1 || !kDirect, "groups read their interleaved copies");
   const int scan = L.scans ? find_scan(L.prefix, L.nscans, unit) : 0;
   const ScanDev &S = scan_of(L, scan);
   if (!S.line) return;  // fan_fp_body's
@@ -445,7 +442,6 @@ __device__ __forceinline__ void line_fp_body(const Launch &L, const int unit) {
   const int view = g < ng ? 4 * vq + 2 * (lw & 1) + ((lane >> 2) & 1) : S.nviews;
   const int det = (ng / 2 + ((g & 1) ? -((g + 1) >> 1) : g >> 1)) * 32 + (lw & 2) * 8 + (lane >> 3) * 4 + (lane & 3);
   const bool valid = view < S.nviews && det < S.ndets;
-  const float *__restrict__ img = S.buf[L.in_buf];
   const T *__restrict__ pk = reinterpret_cast<const T *>(S.pack);
   const LineRay ray = valid ? load_line(S.line + (size_t)view * S.ndets + det) : line_none();
   LineWalk<G> w;
@@ -456,9 +452,6 @@ __device__ __forceinline__ void line_fp_body(const Launch &L, const int unit) {
   const int c0 = none ? -kLinePad : line_c0(ray, n, line_pitch(n));
   const int row0 = none ? 0 : (swap ? n * pitch : 0) + (down ? (n - 1) * pitch : 0);
   const int stride = none ? 0 : down ? -pitch : pitch;
-  // kDirect: rows and columns of the image itself
-  const int drow0 = down ? (n - 1) * (swap ? 1 : n) : 0, dstride = (swap ? 1 : n) * (down ? -1 : 1), dcol = swap ? n : 1;
-  auto direct = [&](int step, int c) { return (unsigned)c < (unsigned)n ? __ldg(img + drow0 + step * dstride + c * dcol) : 0.f; };
   // blocks, from the first any lane has to the last
   const int blk0 = (int)__reduce_min_sync(0xffffffffu, none ? 0xffffu : (unsigned)w.first >> 5);
   const int blk1 = (int)__reduce_max_sync(0xffffffffu, none ? 0u : (unsigned)(w.last >> 5) + 1u);
@@ -468,48 +461,43 @@ __device__ __forceinline__ void line_fp_body(const Launch &L, const int unit) {
   constexpr int kBatch = G;
   auto walk_block = [&](int step0) {
     int c = c0 + w.enter(step0, n);
-    if constexpr (kDirect) {
-      for (int b = 0; b < min(32, n - step0); b++)
-        c += w.row((float)b, direct(step0 + b, c), direct(step0 + b, c + 1)) ? 1 : 0;
+    int off = row0 + step0 * stride;  // the step's row
+    const bool in = none || (w.first <= step0 && step0 + 31 <= w.last);
+    // a column's place in its row; any off the grid (as a line is before and
+    // behind its rows) reads the zeros beside the last one
+    auto any_column = [&](int col) { return (int)min((unsigned)(col + kLinePad), (unsigned)(n + kLinePad + 1)); };
+    // rows b..b+kBatch-1: inside, off is the pixel; else the row
+    auto rows = [&](int b, auto inside) {
+      float f[kBatch];
+      bool x[kBatch];
+      T va[kBatch], vc[kBatch];
+#pragma unroll
+      for (int i = 0; i < kBatch; i++) {
+        f[i] = w.before((float)(b + i));
+        const int at = inside ? off : off + any_column(c);
+        va[i] = __ldg(pk + at);
+        vc[i] = __ldg(pk + at + 1);
+        x[i] = w.crosses((float)(b + i));
+        if (inside) off += x[i] ? 1 : 0;
+        else c += x[i] ? 1 : 0;
+        off += stride;
+      }
+#pragma unroll
+      for (int i = 0; i < kBatch; i++)
+        w.add(f[i], x[i], va[i], vc[i]);
+    };
+    if (__all_sync(0xffffffffu, in)) {
+      off += c + kLinePad;
+#pragma unroll
+      for (int b = 0; b < 32; b += kBatch) rows(b, std::true_type{});
+    } else if (step0 + 32 <= n) {
+#pragma unroll
+      for (int b = 0; b < 32; b += kBatch) rows(b, std::false_type{});
     } else {
-      int off = row0 + step0 * stride;  // the step's row
-      const bool in = none || (w.first <= step0 && step0 + 31 <= w.last);
-      // a column's place in its row; any off the grid (as a line is before and
-      // behind its rows) reads the zeros beside the last one
-      auto any_column = [&](int col) { return (int)min((unsigned)(col + kLinePad), (unsigned)(n + kLinePad + 1)); };
-      // rows b..b+kBatch-1: inside, off is the pixel; else the row
-      auto rows = [&](int b, auto inside) {
-        float f[kBatch];
-        bool x[kBatch];
-        T va[kBatch], vc[kBatch];
-#pragma unroll
-        for (int i = 0; i < kBatch; i++) {
-          f[i] = w.before((float)(b + i));
-          const int at = inside ? off : off + any_column(c);
-          va[i] = __ldg(pk + at);
-          vc[i] = __ldg(pk + at + 1);
-          x[i] = w.crosses((float)(b + i));
-          if (inside) off += x[i] ? 1 : 0;
-          else c += x[i] ? 1 : 0;
-          off += stride;
-        }
-#pragma unroll
-        for (int i = 0; i < kBatch; i++)
-          w.add(f[i], x[i], va[i], vc[i]);
-      };
-      if (__all_sync(0xffffffffu, in)) {
-        off += c + kLinePad;
-#pragma unroll
-        for (int b = 0; b < 32; b += kBatch) rows(b, std::true_type{});
-      } else if (step0 + 32 <= n) {
-#pragma unroll
-        for (int b = 0; b < 32; b += kBatch) rows(b, std::false_type{});
-      } else {
-        for (int b = 0; b < n - step0; b++) {
-          const int at = off + any_column(c);
-          c += w.row((float)b, __ldg(pk + at), __ldg(pk + at + 1)) ? 1 : 0;
-          off += stride;
-        }
+      for (int b = 0; b < n - step0; b++) {
+        const int at = off + any_column(c);
+        c += w.row((float)b, __ldg(pk + at), __ldg(pk + at + 1)) ? 1 : 0;
+        off += stride;
       }
     }
   };
@@ -531,8 +519,7 @@ __device__ __forceinline__ void line_fp_body(const Launch &L, const int unit) {
     s0[m] = ff_zero();
     if (!valid || !((act >> m) & 1u)) continue;
     const float out = tot[m].finish(end, S.lcorr, [&](int p) {
-      if constexpr (kDirect) return __ldg(img + p);
-      else return __ldg(reinterpret_cast<const float *>(pk + (p / n) * pitch + kLinePad + p % n) + m);
+      return __ldg(reinterpret_cast<const float *>(pk + (p / n) * pitch + kLinePad + p % n) + m);
     });
     fp_epilogue(*M[m], L, view * S.ndets + det, out, s0[m]);
   }
@@ -548,21 +535,25 @@ __device__ __forceinline__ void line_fp_body(const Launch &L, const int unit) {
 template <int G>
 __global__ void __launch_bounds__(128) line_fp_kernel(const Launch L) {
   chain_begin();
-  line_fp_body<G, false>(L, blockIdx.x);
+  line_fp_body<G>(L, blockIdx.x);
 }
-__global__ void __launch_bounds__(512) line_fp_direct_kernel(const Launch L) { line_fp_body<1, true>(L, blockIdx.x); }
+// the same in CTAs of sixteen warps, for a launch that must not have many
+__global__ void __launch_bounds__(512) line_fp_wide_kernel(const Launch L) {
+  chain_begin();
+  line_fp_body<1>(L, blockIdx.x);
+}
 template <int G>
 __global__ void __launch_bounds__(128) line_fp_queue_kernel(const Launch L) {
-  persistent_loop(L, [&](int unit) { line_fp_body<G, false>(L, unit); });
+  persistent_loop(L, [&](int unit) { line_fp_body<G>(L, unit); });
 }
 // Scans alone, pairs and larger groups in one launch, whose CTAs fill each
 // other's last waves (a batch of seven 256^2 slices in a three, a pair and two
 // alone: 160 -> 86 us a forward projection).
 __device__ __forceinline__ void line_fp_any_body(const Launch &L, int unit) {
   const int nm = L.scans[find_scan(L.prefix, L.nscans, unit)].nmem;
-  if (nm >= 3) line_fp_body<kGroupMax, false>(L, unit);
-  else if (nm == 2) line_fp_body<2, false>(L, unit);
-  else line_fp_body<1, false>(L, unit);
+  if (nm >= 3) line_fp_body<kGroupMax>(L, unit);
+  else if (nm == 2) line_fp_body<2>(L, unit);
+  else line_fp_body<1>(L, unit);
 }
 __global__ void __launch_bounds__(128, 7) line_fp_any_kernel(const Launch L) {
   chain_begin();
@@ -1276,14 +1267,6 @@ int launch_fp_walk(const Launch &L, int rpt, int nctas, cudaStream_t st) {
   return forms == 3 ? 2 : 1;
 }
 
-// CTAs of a forward projection without copies of the image, with `threads` threads each
-int fp_direct_ctas(const ScanDev &S, int threads) { return line_ctas(S, threads); }
-
-cudaError_t launch_fp_direct(const Launch &L, int threads, cudaStream_t st) {
-  line_fp_direct_kernel<<<fp_direct_ctas(L.single, threads), threads, 0, st>>>(L);
-  return cudaGetLastError();
-}
-
 cudaError_t launch_fp(const Launch &L, int kind, int rpt, int nctas, cudaStream_t st) {
   if (kind == AT_GEOM_GOLDNC) {
     gc_fp_kernel<<<nctas, 128, 0, st>>>(L);
@@ -1342,10 +1325,13 @@ int launch_fp_group(const Launch &L, const Launch &Lpix, const Launch &L1, const
 
 // The row-major and transposed copies of an n x n image that the forward
 // projectors read (lpitch and lpad as in ScanDev), through 32 x 32 shared-memory
-// tiles (coalesced reads and writes)
+// tiles (coalesced reads and writes).  ctl, where given, is cleared on the way
+// (a clear of its own took 2 us of a small call).
 __global__ void __launch_bounds__(256) pack_single_kernel(const float *__restrict__ in, float *__restrict__ out,
-                                                           int n, int pitch, int pad) {
+                                                           int n, int pitch, int pad, Ctl *ctl) {
   in += chain_begin();
+  if (ctl && blockIdx.x + blockIdx.y == 0 && threadIdx.y == 0)
+    for (int i = threadIdx.x; i < (int)(sizeof(Ctl) / sizeof(int)); i += 32) reinterpret_cast<int *>(ctl)[i] = 0;
   __shared__ float t[32][33];
   const int bx = blockIdx.x * 32, by = blockIdx.y * 32;
   float *outt = out + (size_t)n * pitch;
@@ -1374,6 +1360,26 @@ size_t fp_single_scratch_bytes(const Plan &p) {
   return ((sizeof(float) * 2 * (size_t)p.n * pitch + 255) & ~(size_t)255) + sizeof(CUtensorMap);
 }
 
+cudaError_t launch_pack_single(const ScanDev &S, int in_buf, float *copies, Ctl *ctl, cudaStream_t st) {
+  const int nt = (S.n + 31) / 32;
+  return launch_dependent(pack_single_kernel, dim3(nt, nt), dim3(32, 8), 0, st, S.buf[in_buf], copies, S.n, S.lpitch,
+                          S.lpad, ctl);
+}
+
+// CTAs of launch_fp_lines, with `threads` (128 or 512) threads each
+int fp_lines_ctas(const ScanDev &S, int threads) { return line_ctas(S, threads); }
+
+// One forward projection along lines, the image's copies in `copies`
+// (fp_single_scratch_bytes); its control block is cleared first.
+cudaError_t launch_fp_lines(const Launch &L, int threads, float *copies, cudaStream_t st) {
+  const cudaError_t e = launch_pack_single(L.single, L.in_buf, copies, L.single.ctl, st);
+  if (e != cudaSuccess) return e;
+  Launch Lt = L;
+  Lt.single.pack = reinterpret_cast<float4 *>(copies);
+  return launch_dependent(threads == 512 ? line_fp_wide_kernel : line_fp_kernel<1>, fp_lines_ctas(L.single, threads),
+                          threads, 0, st, Lt);
+}
+
 // One fan-beam / ray-table forward projection outside a batch: the image's
 // row-major and transposed copies into `scratch` (fp_single_scratch_bytes),
 // then the slab projector when the plan has slab tables, else the L1 walk.
@@ -1383,8 +1389,7 @@ cudaError_t launch_fp_single(const Launch &L, const Plan &p, int rpt, void *scra
   const ScanDev &S = L.single;
   const int n = S.n;
   float *copies = reinterpret_cast<float *>(scratch);
-  cudaError_t e = launch_dependent(pack_single_kernel, dim3((n + 31) / 32, (n + 31) / 32), dim3(32, 8), 0, st,
-                                   S.buf[L.in_buf], copies, n, S.lpitch, S.lpad);
+  cudaError_t e = launch_pack_single(S, L.in_buf, copies, nullptr, st);
   if (e != cudaSuccess) return e;
   Launch Lt = L;
   Lt.single.pack = reinterpret_cast<float4 *>(copies);
