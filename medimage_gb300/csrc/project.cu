@@ -417,7 +417,7 @@ __global__ void __launch_bounds__(128) fan_fp_queue_kernel(const Launch L) {
 // L1 at C2), the L1 data path for four (84 %: 2 x 16 bytes a row and lane).
 // C2, the image's copies included: one slice 243 -> 130 us, eight slices
 // 812 -> 560 us; error against 64 bits 2.2e-7 -> 1.3e-7.
-template <int G>
+template <int G, int kBatch = 2>
 __device__ __forceinline__ void line_fp_body(const Launch &L, const int unit) {
   using T = typename Elem<G>::T;
   const int scan = L.scans ? find_scan(L.prefix, L.nscans, unit) : 0;
@@ -456,9 +456,9 @@ __device__ __forceinline__ void line_fp_body(const Launch &L, const int unit) {
   const int blk0 = (int)__reduce_min_sync(0xffffffffu, none ? 0xffffu : (unsigned)w.first >> 5);
   const int blk1 = (int)__reduce_max_sync(0xffffffffu, none ? 0u : (unsigned)(w.last >> 5) + 1u);
   // Rows are taken kBatch at a time: the crossings and the pixels first (the
-  // crossings need none), then the sums.  One to four rows measure within 3 %
-  // of each other.
-  constexpr int kBatch = G;
+  // crossings need none), then the sums.  One to four measure within 3 % of each
+  // other: two, but four for launches of larger groups alone (eight slices of
+  // 512^2 548 -> 542 us; a four beside one alone 380 -> 389 us).
   auto walk_block = [&](int step0) {
     int c = c0 + w.enter(step0, n);
     int off = row0 + step0 * stride;  // the step's row
@@ -473,11 +473,12 @@ __device__ __forceinline__ void line_fp_body(const Launch &L, const int unit) {
       T va[kBatch], vc[kBatch];
 #pragma unroll
       for (int i = 0; i < kBatch; i++) {
-        f[i] = w.before((float)(b + i));
+        w.at(b + i);
+        f[i] = w.before(b + i);
         const int at = inside ? off : off + any_column(c);
         va[i] = __ldg(pk + at);
         vc[i] = __ldg(pk + at + 1);
-        x[i] = w.crosses((float)(b + i));
+        x[i] = w.crosses(b + i);
         if (inside) off += x[i] ? 1 : 0;
         else c += x[i] ? 1 : 0;
         off += stride;
@@ -496,7 +497,7 @@ __device__ __forceinline__ void line_fp_body(const Launch &L, const int unit) {
     } else {
       for (int b = 0; b < n - step0; b++) {
         const int at = off + any_column(c);
-        c += w.row((float)b, __ldg(pk + at), __ldg(pk + at + 1)) ? 1 : 0;
+        c += w.row(b, __ldg(pk + at), __ldg(pk + at + 1)) ? 1 : 0;
         off += stride;
       }
     }
@@ -535,7 +536,14 @@ __device__ __forceinline__ void line_fp_body(const Launch &L, const int unit) {
 template <int G>
 __global__ void __launch_bounds__(128) line_fp_kernel(const Launch L) {
   chain_begin();
-  line_fp_body<G>(L, blockIdx.x);
+  line_fp_body<G, G == kGroupMax ? 4 : 2>(L, blockIdx.x);
+}
+// One member with 64 registers, not the compiler's 56: more pixels in flight
+// (512^2 132 -> 126 us, four views of it 44 -> 38 us).
+template <>
+__global__ void __launch_bounds__(128, 8) line_fp_kernel<1>(const Launch L) {
+  chain_begin();
+  line_fp_body<1>(L, blockIdx.x);
 }
 // the same in CTAs of sixteen warps, for a launch that must not have many
 __global__ void __launch_bounds__(512) line_fp_wide_kernel(const Launch L) {

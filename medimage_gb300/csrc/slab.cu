@@ -138,11 +138,12 @@ __global__ void __launch_bounds__(512, 2) fan_fp_slab_kernel(const Launch L) {
       for (int r = lw.first & ~31; r <= lw.last; r++) {
         if ((r & 31) == 0) lcol = lcol0 + lw.enter(r, S.n);
         if (r < lw.first) {  // not in the grid yet
-          lcol += lw.crosses((float)(r & 31)) ? 1 : 0;
+          lw.at(r & 31);
+          lcol += lw.crosses(r & 31) ? 1 : 0;
           continue;
         }
         const T *row = copy + line_row_of(ray, r, S.n) * S.lpitch;
-        lcol += lw.row((float)(r & 31), __ldg(row + lcol), __ldg(row + lcol + 1)) ? 1 : 0;
+        lcol += lw.row(r & 31, __ldg(row + lcol), __ldg(row + lcol + 1)) ? 1 : 0;
         if (r == lw.last || (r & 31) == 31)
 #pragma unroll
           for (int m = 0; m < G; m++) tot[m].fold(lw.part[m]);
@@ -229,11 +230,14 @@ __global__ void __launch_bounds__(512, 2) fan_fp_slab_kernel(const Launch L) {
                           __ldg(wlo_row + s) + ((dir > 0 ? r0 : S.n - 1 - r0) - u0) * WB;
           if (r0 == lw.first) {  // the block's steps before the grid
             lcol = lcol0 + lw.enter(r0 & ~31, S.n);
-            for (int r = r0 & ~31; r < r0; r++) lcol += lw.crosses((float)(r & 31)) ? 1 : 0;
+            for (int r = r0 & ~31; r < r0; r++) {
+              lw.at(r & 31);
+              lcol += lw.crosses(r & 31) ? 1 : 0;
+            }
           }
           for (int r = r0; r <= r1; r++, tile += dir * WB) {
             if ((r & 31) == 0) lcol = lcol0 + lw.enter(r, S.n);
-            lcol += lw.row((float)(r & 31), tile[lcol], tile[lcol + 1]) ? 1 : 0;
+            lcol += lw.row(r & 31, tile[lcol], tile[lcol + 1]) ? 1 : 0;
             if (r == lw.last || (r & 31) == 31)
 #pragma unroll
               for (int m = 0; m < G; m++) tot[m].fold(lw.part[m]);
@@ -543,12 +547,13 @@ __global__ void slab_extent_kernel(int n, int nviews, int ndets, int nbpv, int v
     for (int k = w.first & ~31; k <= w.last; k++) {
       if ((k & 31) == 0) col = col0 + w.enter(k, n);
       if (k < w.first) {
-        col += w.crosses((float)(k & 31)) ? 1 : 0;
+        w.at(k & 31);
+        col += w.crosses(k & 31) ? 1 : 0;
         continue;
       }
       mn = min(mn, col);
       mx = max(mx, col + 1);
-      col += w.row((float)(k & 31), 0.f, 0.f) ? 1 : 0;
+      col += w.row(k & 31, 0.f, 0.f) ? 1 : 0;
       const int u = line_row_of(r, k, n), next = (r.flags & kLineDown) ? u - 1 : u + 1;
       if (k == w.last || next / rows != u / rows) {
         atomicMin(lo + (size_t)cta * nslab + u / rows, mn);

@@ -104,7 +104,7 @@ __device__ __forceinline__ int strip_scale_exp(const ScanDev &S, float mx) {
   return min(S.bp_term_bits - ex, 120);
 }
 
-// One row of a ray for M members (LineWalk's before() and crosses()): the part
+// One row of a ray for M members (LineWalk's at(), before() and crosses()): the part
 // before the crossing to the pixel at addr, rounded by kMagic, and where the
 // ray crosses the rest of the rounded whole to the next pixel; then on to the
 // next row.  Without a crossing the rest is zero: one member adds it all the
@@ -114,10 +114,12 @@ __device__ __forceinline__ int strip_scale_exp(const ScanDev &S, float mx) {
 // wavefronts (four slices 612 us against 682).  kChecked: adds to columns
 // outside the strip (col, of ncols) are left out.
 template <int M, int kPlane, bool kChecked>
-__device__ __forceinline__ void strip_row(float &e, unsigned &addr, int &col, int ncols, float inv, int step, float b,
+__device__ __forceinline__ void strip_row(float &e, unsigned &addr, int &col, int ncols, float inv, int step, int b,
                                           const float (&rs)[M], const int (&whole)[M]) {
-  const float f = __saturatef(e + (16.f - b));
-  const bool x = e < b - 15.f;
+  constexpr int kSub = LineWalk<1>::kSub;
+  if (b > 0 && b % kSub == 0) e -= (float)kSub;
+  const float f = __saturatef(e - (float)(b % kSub - kSub / 2));
+  const bool x = e < (float)(b % kSub + 1 - kSub / 2);
   int bits[M];
 #pragma unroll
   for (int m = 0; m < M; m++) bits[m] = __float_as_int(fmaf(f, rs[m], kMagic));
@@ -147,7 +149,7 @@ __device__ __forceinline__ void strip_walk(const LineWalk<1> &w, unsigned addr, 
   float e = w.e;
 #pragma unroll
   for (int b = 0; b < kStripCellRows; b++)
-    strip_row<M, kPlane, kChecked>(e, addr, col, ncols, w.inv, step, (float)b, rs, whole);
+    strip_row<M, kPlane, kChecked>(e, addr, col, ncols, w.inv, step, b, rs, whole);
 }
 
 template <int G>
@@ -526,7 +528,10 @@ __global__ void strip_range_kernel(int n, int nviews, int ndets, int ncr, int nc
     if (w.last < step0 || w.first >= step0 + kStripCellRows) continue;
     const int c0 = col0 + w.enter(step0, n);
     int c1 = c0;
-    for (int b = 0; b < kStripCellRows; b++) c1 += w.crosses((float)b) ? 1 : 0;
+    for (int b = 0; b < kStripCellRows; b++) {
+      w.at(b);
+      c1 += w.crosses(b) ? 1 : 0;
+    }
     // one more on either side: a taller strip's walk enters at its own first row
     const int lo = max(c0 - 1, 0), hi = min(c1 + 2, n - 1);
     if (lo > hi) continue;
@@ -564,8 +569,9 @@ __global__ void strip_hits_kernel(int n, int view0, int view1, int ndets, int nc
     if (w.last < step0 || w.first >= step0 + kStripCellRows) continue;
     int c = col0 + w.enter(step0, n);
     for (int b = 0; b < kStripCellRows; b++) {
-      const float f = w.before((float)b);
-      const bool x = w.crosses((float)b);
+      w.at(b);
+      const float f = w.before(b);
+      const bool x = w.crosses(b);
       const int u = line_row_of(r, step0 + b, n);
       add(u, c, f);
       if (x) add(u, ++c, 1.f - f);
