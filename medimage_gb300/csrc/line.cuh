@@ -115,29 +115,24 @@ struct LineWalk {
     if (x) fma_elem<G>(part, 1.f - f, c);
   }
   __device__ __forceinline__ bool row(int b, const typename Elem<G>::T &a, const typename Elem<G>::T &c) {
-    at(b);
     const float f = before(b);
     const bool x = crosses(b);
     add(f, x, a, c);
     return x;
   }
+  // a block's step of any number: enter() or at(), as it needs; col: the column,
+  // which enter() sets
+  __device__ __forceinline__ void to(int step, int n, int c0, int &col) {
+    if (step % kSub != 0) return;
+    if ((step & 31) == 0) col = c0 + enter(step, n);
+    else at(step & 31);
+  }
 };
 
-// the Kahan total of a ray's block sums for one scan, and its line integral
+// the Kahan total of a ray's block sums for one scan
 struct LineTotal {
   float acc = 0.f, comp = 0.f;
   __device__ __forceinline__ void fold(float part) { kahan_add(acc, comp, part); }
-  // with the ray's corrections: value(pixel) reads the scan's pixel x*n + y
-  template <typename V>
-  __device__ __forceinline__ float finish(const LineRay &r, const LineCorr *__restrict__ corr, V &&value) const {
-    float out = (acc - comp) * r.len;
-    const int nc = (int)(r.flags >> 8);
-    for (int k = 0; k < nc; k++) {
-      const LineCorr c = corr[r.corr0 + k];
-      out = fmaf(c.w, value(c.pix & ~kCorrForwardOnly), out);
-    }
-    return out;
-  }
 };
 
 // column c0, and the first element of a step's row in its copy
@@ -170,6 +165,94 @@ __device__ __forceinline__ LineRay load_line(const LineRay *p) {
   r.corr0 = (int)b.z;
   r.flags = b.w;
   return r;
+}
+
+template <int G>
+__device__ __forceinline__ float elem_of(const typename Elem<G>::T &v, int m) {
+  if constexpr (G == 1) return v;
+  else if constexpr (G == 2) return m == 0 ? v.x : v.y;
+  else return m == 0 ? v.x : m == 1 ? v.y : m == 2 ? v.z : v.w;
+}
+
+// The sum along a line without the pixels of its corrections, from one scan's
+// values (every stride-th float of the copies at pk): the walk again, pixel by
+// pixel, of the rows in the grid and the parts that are not empty.
+__device__ __forceinline__ float line_sum_without(const float *pk, int stride, const LineRay *rayp, const LineCorr *corr,
+                                                  int n, int pitch) {
+  const LineRay r = load_line(rayp);
+  const bool swap = (r.flags & kLineSwap) != 0;
+  const int nc = (int)(r.flags >> 8), col0 = line_c0(r, n, pitch);
+  LineWalk<1> w;
+  w.load(r);
+  LineTotal tot;
+  int col = 0;
+  for (int step = w.first & ~31; step <= w.last; step++) {
+    w.to(step, n, col0, col);
+    const float f = w.before(step & 31);
+    const bool x = w.crosses(step & 31);
+    const int u = line_row_of(r, step, n);
+    for (int k = 0; k < 2 && step >= w.first; k++) {
+      const int c = col + k;
+      const float part = k == 0 ? f : x ? 1.f - f : 0.f;
+      bool use = part > 0.f && (unsigned)c < (unsigned)n;
+      for (int i = 0; i < nc; i++) use = use && corr[r.corr0 + i].pix != (swap ? c * n + u : u * n + c);
+      if (use) w.part[0] = fmaf(part, pk[(size_t)stride * ((swap ? n * pitch : 0) + u * pitch + kLinePad + c)], w.part[0]);
+    }
+    col += x ? 1 : 0;
+    if (step == w.last || (step & 31) == 31) tot.fold(w.part[0]);
+  }
+  return (tot.acc - tot.comp) * r.len;
+}
+
+// The G scans' line integrals of a warp's rays, with their corrections, from the
+// padded copies at pk.  A ray that is no line is its corrections.
+// A line's corrections are the last pieces that the traversal leaves out, as
+// minus what the line had: where that leaves little or nothing of the sum
+// (their pixels not finite, or far above the others), the line is walked again
+// without them (inlined: a call cost every walk 2 % of its registers' schedule).
+template <int G>
+__device__ __forceinline__ void line_finish(const LineRay *rayp, bool valid, const LineCorr *__restrict__ corr,
+                                            const LineTotal (&tot)[G],
+                                            const typename Elem<G>::T *__restrict__ pk, int n, int pitch,
+                                            float (&out)[G]) {
+  const LineRay r = valid ? load_line(rayp) : line_none();
+  const int nc = (int)(r.flags >> 8);
+  const bool whole = (r.rows & 0xffffu) > r.rows >> 16;
+  // pixel x*n + y in the row-major copy: x rows' padding further on
+  const float rcp = __frcp_rn((float)n);
+  auto value = [&](int pix) {
+    const int p = pix & ~kCorrForwardOnly;
+    int x = (int)((float)p * rcp);
+    const int y = p - x * n;  // (x is one off at most: p is below 2^26)
+    x += y >= n ? 1 : y < 0 ? -1 : 0;
+    return __ldg(pk + p + x * (pitch - n) + kLinePad);
+  };
+  bool again = false;
+#pragma unroll
+  for (int m = 0; m < G; m++) out[m] = (tot[m].acc - tot[m].comp) * r.len;
+  if (nc > 0) {
+    float line[G];
+#pragma unroll
+    for (int m = 0; m < G; m++) line[m] = out[m];
+    for (int k = 0; k < nc; k++) {
+      const LineCorr c = corr[r.corr0 + k];
+      const typename Elem<G>::T v = value(c.pix);
+#pragma unroll
+      for (int m = 0; m < G; m++) out[m] = fmaf(c.w, elem_of<G>(v, m), out[m]);
+    }
+#pragma unroll
+    for (int m = 0; m < G; m++) again |= !whole && !(fabsf(line[m]) <= 1024.f * fabsf(out[m]));
+    if (again)
+#pragma unroll 1
+      for (int m = 0; m < G; m++) {
+        const float o = m == 0 ? out[0] : m == 1 ? out[G > 1 ? 1 : 0] : m == 2 ? out[G > 2 ? 2 : 0] : out[G - 1];
+        const float l = m == 0 ? line[0] : m == 1 ? line[G > 1 ? 1 : 0] : m == 2 ? line[G > 2 ? 2 : 0] : line[G - 1];
+        if (fabsf(l) <= 1024.f * fabsf(o)) continue;
+        const float s = line_sum_without(reinterpret_cast<const float *>(pk) + m, G, rayp, corr, n, pitch);
+#pragma unroll
+        for (int j = 0; j < G; j++) out[j] = j == m ? s : out[j];
+      }
+  }
 }
 
 }  // namespace medimg

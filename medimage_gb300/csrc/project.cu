@@ -456,9 +456,9 @@ __device__ __forceinline__ void line_fp_body(const Launch &L, const int unit) {
   const int blk0 = (int)__reduce_min_sync(0xffffffffu, none ? 0xffffu : (unsigned)w.first >> 5);
   const int blk1 = (int)__reduce_max_sync(0xffffffffu, none ? 0u : (unsigned)(w.last >> 5) + 1u);
   // Rows are taken kBatch at a time: the crossings and the pixels first (the
-  // crossings need none), then the sums.  One to four measure within 3 % of each
-  // other: two, but four for launches of larger groups alone (eight slices of
-  // 512^2 548 -> 542 us; a four beside one alone 380 -> 389 us).
+  // crossings need none), then the sums.  Launches of one form four (with two,
+  // one slice of 1024^2 717 us for 702, a pair of 512^2 160 us for 152), mixed ones
+  // two (with four, a four beside one alone 389 us for 380).
   auto walk_block = [&](int step0) {
     int c = c0 + w.enter(step0, n);
     int off = row0 + step0 * stride;  // the step's row
@@ -497,6 +497,7 @@ __device__ __forceinline__ void line_fp_body(const Launch &L, const int unit) {
     } else {
       for (int b = 0; b < n - step0; b++) {
         const int at = off + any_column(c);
+        w.at(b);
         c += w.row(b, __ldg(pk + at), __ldg(pk + at + 1)) ? 1 : 0;
         off += stride;
       }
@@ -513,16 +514,17 @@ __device__ __forceinline__ void line_fp_body(const Launch &L, const int unit) {
 #pragma unroll
   for (int m = 0; m < G; m++) M[m] = L.scans ? &L.scans[S.mem[(act >> m) & 1u ? m : 0]] : &L.single;
   const int ncta = L.scans ? __ldg(L.prefix + scan + 1) - cta0 : gridDim.x;
-  const LineRay end = valid ? load_line(S.line + (size_t)view * S.ndets + det) : line_none();
+  // (what the end needs is computed there: ahead of the walk it would hold
+  // registers through it; 1024^2 722 -> 717 us)
+  float out[G];
+  int n_end = n, view_end = view;
+  asm volatile("" : "+r"(n_end), "+r"(view_end) : : "memory");
+  line_finish<G>(S.line + (size_t)view_end * S.ndets + det, valid, S.lcorr, tot, pk, n_end, line_pitch(n_end), out);
   FF s0[G];
 #pragma unroll
   for (int m = 0; m < G; m++) {
     s0[m] = ff_zero();
-    if (!valid || !((act >> m) & 1u)) continue;
-    const float out = tot[m].finish(end, S.lcorr, [&](int p) {
-      return __ldg(reinterpret_cast<const float *>(pk + (p / n) * pitch + kLinePad + p % n) + m);
-    });
-    fp_epilogue(*M[m], L, view * S.ndets + det, out, s0[m]);
+    if (valid && ((act >> m) & 1u)) fp_epilogue(*M[m], L, view * S.ndets + det, out[m], s0[m]);
   }
   if (stage_reduces(L.stage)) {
     if constexpr (G == 1) {
@@ -533,17 +535,14 @@ __device__ __forceinline__ void line_fp_body(const Launch &L, const int unit) {
   }
 }
 
+// 64 registers for one member and for two (56 for one, the compiler's choice
+// once: 512^2 132 us for 126, four views of it 44 us for 38; 72: 129 us), 72 for four.
 template <int G>
-__global__ void __launch_bounds__(128) line_fp_kernel(const Launch L) {
+constexpr int kLineCtas = G == kGroupMax ? 7 : 8;
+template <int G>
+__global__ void __launch_bounds__(128, kLineCtas<G>) line_fp_kernel(const Launch L) {
   chain_begin();
-  line_fp_body<G, G == kGroupMax ? 4 : 2>(L, blockIdx.x);
-}
-// One member with 64 registers, not the compiler's 56: more pixels in flight
-// (512^2 132 -> 126 us, four views of it 44 -> 38 us).
-template <>
-__global__ void __launch_bounds__(128, 8) line_fp_kernel<1>(const Launch L) {
-  chain_begin();
-  line_fp_body<1>(L, blockIdx.x);
+  line_fp_body<G, 4>(L, blockIdx.x);
 }
 // the same in CTAs of sixteen warps, for a launch that must not have many
 __global__ void __launch_bounds__(512) line_fp_wide_kernel(const Launch L) {
@@ -551,7 +550,7 @@ __global__ void __launch_bounds__(512) line_fp_wide_kernel(const Launch L) {
   line_fp_body<1>(L, blockIdx.x);
 }
 template <int G>
-__global__ void __launch_bounds__(128) line_fp_queue_kernel(const Launch L) {
+__global__ void __launch_bounds__(128, kLineCtas<G>) line_fp_queue_kernel(const Launch L) {
   persistent_loop(L, [&](int unit) { line_fp_body<G>(L, unit); });
 }
 // Scans alone, pairs and larger groups in one launch, whose CTAs fill each

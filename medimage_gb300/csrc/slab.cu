@@ -136,9 +136,8 @@ __global__ void __launch_bounds__(512, 2) fan_fp_slab_kernel(const Launch L) {
     if constexpr (kLine) {
       const T *copy = pack + (ray.off - lcol0);
       for (int r = lw.first & ~31; r <= lw.last; r++) {
-        if ((r & 31) == 0) lcol = lcol0 + lw.enter(r, S.n);
+        lw.to(r, S.n, lcol0, lcol);
         if (r < lw.first) {  // not in the grid yet
-          lw.at(r & 31);
           lcol += lw.crosses(r & 31) ? 1 : 0;
           continue;
         }
@@ -229,14 +228,13 @@ __global__ void __launch_bounds__(512, 2) fan_fp_slab_kernel(const Launch L) {
           const T *tile = reinterpret_cast<const T *>(buf_base + (i & 1) * buf_bytes) -
                           __ldg(wlo_row + s) + ((dir > 0 ? r0 : S.n - 1 - r0) - u0) * WB;
           if (r0 == lw.first) {  // the block's steps before the grid
-            lcol = lcol0 + lw.enter(r0 & ~31, S.n);
             for (int r = r0 & ~31; r < r0; r++) {
-              lw.at(r & 31);
+              lw.to(r, S.n, lcol0, lcol);
               lcol += lw.crosses(r & 31) ? 1 : 0;
             }
           }
           for (int r = r0; r <= r1; r++, tile += dir * WB) {
-            if ((r & 31) == 0) lcol = lcol0 + lw.enter(r, S.n);
+            lw.to(r, S.n, lcol0, lcol);
             lcol += lw.row(r & 31, tile[lcol], tile[lcol + 1]) ? 1 : 0;
             if (r == lw.last || (r & 31) == 31)
 #pragma unroll
@@ -337,23 +335,16 @@ __global__ void __launch_bounds__(512, 2) fan_fp_slab_kernel(const Launch L) {
   FF s0[G];
 #pragma unroll
   for (int m = 0; m < G; m++) s0[m] = ff_zero();
-  if (valid) {
-    const int bin = view * S.ndets + det;
-    float out[G];
-    if constexpr (kLine) {
+  float out[G];
+  if constexpr (kLine) {
+    line_finish<G>(S.line + (size_t)view * S.ndets + det, valid, S.lcorr, tot, pack, S.n, S.lpitch, out);
+  } else {
 #pragma unroll
-      for (int m = 0; m < G; m++)
-        out[m] = tot[m].finish(ray, S.lcorr, [&](int p) {
-          return __ldg(reinterpret_cast<const float *>(pack + (size_t)(p / S.n) * S.lpitch + S.lpad + p % S.n) + m);
-        });
-    } else {
-#pragma unroll
-      for (int m = 0; m < G; m++) out[m] = acc[m] - comp[m];
-    }
-#pragma unroll
-    for (int m = 0; m < G; m++)
-      if (act[m]) fp_epilogue(*M[m], L, bin, out[m], s0[m]);
+    for (int m = 0; m < G; m++) out[m] = acc[m] - comp[m];
   }
+#pragma unroll
+  for (int m = 0; m < G; m++)
+    if (valid && act[m]) fp_epilogue(*M[m], L, view * S.ndets + det, out[m], s0[m]);
   if (stage_reduces(L.stage)) {
     if constexpr (G == 1) {
       reduce_and_finalize<1>(*M[0], L, s0, local_cta, ncta);
@@ -545,9 +536,8 @@ __global__ void slab_extent_kernel(int n, int nviews, int ndets, int nbpv, int v
     const int col0 = line_c0(r, n, line_pitch(n));
     int col = 0, mn = INT_MAX, mx = INT_MIN;
     for (int k = w.first & ~31; k <= w.last; k++) {
-      if ((k & 31) == 0) col = col0 + w.enter(k, n);
+      w.to(k, n, col0, col);
       if (k < w.first) {
-        w.at(k & 31);
         col += w.crosses(k & 31) ? 1 : 0;
         continue;
       }
