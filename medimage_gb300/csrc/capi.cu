@@ -75,7 +75,10 @@ cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t st) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  if (dev >= kMaxDevices) return cudaMallocAsync(p, bytes, st);
+  // under capture the memory becomes the graph's
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if ((e = cudaStreamIsCapturing(st, &capture)) != cudaSuccess) return e;
+  if (dev >= kMaxDevices || capture != cudaStreamCaptureStatusNone) return cudaMallocAsync(p, bytes, st);
   cudaMemPool_t pool;
   {
     ScratchPools &P = scratch_pools();
