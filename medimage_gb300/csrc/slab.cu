@@ -36,6 +36,7 @@
 #include "epilogue.cuh"
 #include "line.cuh"
 #include "mbar.cuh"
+#include "smem_optin.h"
 #include "solver.h"
 
 namespace medimg {
@@ -366,28 +367,23 @@ size_t slab_smem_bytes(int G, int rows, int wbox) {
 }
 
 namespace {
-// Raises the kernel's dynamic shared memory limit to what a launch needs
-// (once per size; the limit is the device's opt-in maximum less the kernel's
-// static shared memory).  Returns cudaErrorInvalidValue for a size beyond it.
+// Raises the kernel's dynamic shared memory limit to what a launch needs (the
+// limit is the device's opt-in maximum less the kernel's static shared memory).
+// Returns cudaErrorInvalidValue for a size beyond it.
 template <int G, bool kLine>
 cudaError_t launch_slab_g(const Launch &L, int nctas, int threads, size_t smem, cudaStream_t st) {
-  static std::mutex mu;
-  static size_t granted = 48 * 1024;  // every kernel may take 48 KB without opting in
-  if (smem > granted) {
-    std::lock_guard<std::mutex> lk(mu);
-    if (smem > granted) {
-      int dev = 0, optin = 0;
-      cudaError_t e = cudaGetDevice(&dev);
-      if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-      cudaFuncAttributes fa{};
-      if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, fan_fp_slab_kernel<G, kLine>);
-      if (e != cudaSuccess) return e;
-      if (smem + fa.sharedSizeBytes > (size_t)optin) return cudaErrorInvalidValue;
-      e = cudaFuncSetAttribute(fan_fp_slab_kernel<G, kLine>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-      granted = smem;
-    }
-  }
+  static SmemOptIn optin;
+  const cudaError_t e = optin.ensure(smem, [](int *dev) { return cudaGetDevice(dev); }, [](size_t bytes) {
+    int dev = 0, most = 0;
+    cudaFuncAttributes fa{};
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, fan_fp_slab_kernel<G, kLine>);
+    if (e != cudaSuccess) return e;
+    if (bytes + fa.sharedSizeBytes > (size_t)most) return cudaErrorInvalidValue;
+    return cudaFuncSetAttribute(fan_fp_slab_kernel<G, kLine>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  });
+  if (e != cudaSuccess) return e;
   fan_fp_slab_kernel<G, kLine><<<nctas, threads, smem, st>>>(L);
   return cudaGetLastError();
 }

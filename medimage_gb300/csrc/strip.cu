@@ -29,7 +29,6 @@
 #include <algorithm>
 #include <climits>
 #include <cmath>
-#include <mutex>
 #include <type_traits>
 #include <utility>
 #include <vector>
@@ -37,6 +36,7 @@
 #include "epilogue.cuh"
 #include "launch.h"
 #include "line.cuh"
+#include "smem_optin.h"
 #include "solver.h"
 
 namespace medimg {
@@ -428,12 +428,11 @@ int strip_cells(const ScanDev &S, int nmem) {
 }  // namespace
 
 cudaError_t launch_strip_bp(const Launch &L, int nctas, cudaStream_t st) {
-  static std::once_flag once;
-  static cudaError_t err = cudaSuccess;
-  std::call_once(once, [] {
-    err = cudaFuncSetAttribute(strip_bp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStripSmem);
+  static SmemOptIn optin;
+  const cudaError_t e = optin.ensure(kStripSmem, [](int *dev) { return cudaGetDevice(dev); }, [](size_t bytes) {
+    return cudaFuncSetAttribute(strip_bp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   });
-  if (err != cudaSuccess) return err;
+  if (e != cudaSuccess) return e;
   return launch_dependent(strip_bp_kernel, nctas, kStripThreads, kStripSmem, st, L);
 }
 
