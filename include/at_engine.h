@@ -168,16 +168,21 @@ int at_plan_create_rays(int32_t n, double pixel_mm, int32_t nviews, int32_t ndet
  * The forward projector of the reference
  * (helical/rebin/src/tracing.cpp:22-147 applied per ray) has no such knob. */
 int at_plan_set_forward_variant(at_plan *plan, int32_t views, int32_t rays, int32_t rows);
-/* Pins the back projector of a fan-beam or ray-table plan, which by default
- * walks the rays as lines (fastest; plans traced in FP32, and ray tables most
- * of whose rays end inside the grid, walk tile runs), for launches of
+/* Pins the back projector of a fan-beam or ray-table plan for launches of
  * single scans (use bit0) and of groups of scans that share the plan (bit1):
  * a set bit gathers each pixel's terms from the plan's pixel table (the
  * traversal stored by pixel and view, with each segment's FP32 weight; built
  * on the first call that asks for it, about 4 bytes per segment plus 4 per
  * pixel and view), a clear bit walks the (ray, 16x16 tile) runs.  Results
- * are bitwise the same either way: both add the same fixed-point terms (the
- * walk along lines rounds a ray's crossings more finely).
+ * are bitwise the same for every mask: all add the same fixed-point terms.
+ * A plan that is not pinned walks its rays as lines, which is faster (512^2,
+ * 720 x 888: 181 us a back projection, tile runs 269, the table 690) and
+ * rounds a ray's crossings more finely, so its sums differ in their last bits;
+ * plans traced in FP32, and ray tables with many rays that end inside the
+ * grid or whose sums along lines could leave the fixed-point range, walk tile
+ * runs by default.  at_plan_reset_back_variant returns a plan to its default
+ * (mask 0 pins tile runs).  at_plan_get_back_variant: -1 while the plan walks
+ * lines, else the mask in use.
  * AT_EINVAL for a mask outside 0..3 or a plan the table's fields cannot hold
  * (more than 32767 detectors, or 63 rays of one view through one pixel).
  * Solvers, projection sets and servers made before the call keep the variant
@@ -186,6 +191,8 @@ int at_plan_set_forward_variant(at_plan *plan, int32_t views, int32_t rays, int3
  * back projector (helical/rebin/src/tracing.cpp:22-147, transposed per ray)
  * has no such knob. */
 int at_plan_set_back_variant(at_plan *plan, int32_t use);
+int at_plan_reset_back_variant(at_plan *plan);
+int at_plan_get_back_variant(const at_plan *plan, int32_t *use);
 void at_plan_destroy(at_plan *plan);
 /* Launch form of the projectors of batches (solvers, projection sets, server
  * groups) made after the call, fan-beam and ray-table plans: 0 = one CTA per

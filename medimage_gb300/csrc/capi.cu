@@ -325,6 +325,25 @@ AT_API int at_plan_set_back_variant(at_plan *plan, int32_t use) {
   return AT_OK;
 }
 
+AT_API int at_plan_reset_back_variant(at_plan *plan) {
+  AT_CHECK_ARG(plan, "at_plan_reset_back_variant: null plan");
+  Plan &p = plan->p;
+  AT_CHECK_ARG(p.kind == AT_GEOM_FAN || p.kind == AT_GEOM_RAYS,
+               "at_plan_reset_back_variant: fan-beam and ray-table plans only");
+  p.bp_table = 0;
+  p.bp_pinned = 0;
+  return AT_OK;
+}
+
+AT_API int at_plan_get_back_variant(const at_plan *plan, int32_t *use) {
+  AT_CHECK_ARG(plan && use, "at_plan_get_back_variant: null argument");
+  const Plan &p = plan->p;
+  AT_CHECK_ARG(p.kind == AT_GEOM_FAN || p.kind == AT_GEOM_RAYS,
+               "at_plan_get_back_variant: fan-beam and ray-table plans only");
+  *use = p.strip_ok && !p.bp_pinned ? -1 : p.pt_meta_d ? p.bp_table : 0;
+  return AT_OK;
+}
+
 AT_API int at_plan_get_stats(const at_plan *plan, at_plan_stats *out) {
   AT_CHECK_ARG(plan && out, "at_plan_get_stats: null argument");
   const Plan &p = plan->p;

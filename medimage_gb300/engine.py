@@ -127,6 +127,8 @@ SIGNATURES = {
     "at_plan_create_goldnc": ([C.POINTER(C.c_void_p)], C.c_int),
     "at_plan_set_forward_variant": ([C.c_void_p, C.c_int32, C.c_int32, C.c_int32], C.c_int),
     "at_plan_set_back_variant": ([C.c_void_p, C.c_int32], C.c_int),
+    "at_plan_reset_back_variant": ([C.c_void_p], C.c_int),
+    "at_plan_get_back_variant": ([C.c_void_p, C.POINTER(C.c_int32)], C.c_int),
     "at_set_batch_launch_mode": ([C.c_int32], C.c_int),
     "at_rowaction_create": ([C.c_int32, C.c_int32, C.c_int32, C.POINTER(C.c_void_p)], C.c_int),
     "at_rowaction_destroy": ([C.c_void_p], None),
@@ -448,8 +450,23 @@ class Plan:
         """Pin the back projector of later batches (by default rays are walked
         as lines): bit0 single scans, bit1 groups of scans sharing the plan
         gather from the pixel table (built on first use); a clear bit walks
-        tile runs.  Bitwise the same sums either way."""
+        tile runs.  Bitwise the same sums for every mask."""
         _check("at_plan_set_back_variant", lib().at_plan_set_back_variant(self._h, use))
+        self._read_stats()
+
+    def reset_back_variant(self) -> None:
+        """Back to the plan's default back projector."""
+        _check("at_plan_reset_back_variant", lib().at_plan_reset_back_variant(self._h))
+        self._read_stats()
+
+    @property
+    def back_variant(self) -> int:
+        """-1 while back projections walk the rays as lines, else the mask of set_back_variant."""
+        use = C.c_int32()
+        _check("at_plan_get_back_variant", lib().at_plan_get_back_variant(self._h, C.byref(use)))
+        return use.value
+
+    def _read_stats(self) -> None:
         st = _PlanStats()
         _check("at_plan_get_stats", lib().at_plan_get_stats(self._h, C.byref(st)))
         self.stats = {k: getattr(st, k) for k, _ in _PlanStats._fields_}
