@@ -214,9 +214,12 @@ int at_plan_trace_ray(const at_plan *plan, int32_t view, int32_t det, int32_t *h
 
 /* ---- projectors (FP32, device buffers) ---- */
 /* d_sino[view][det] = sum over the ray's segments of d_img[pixel] * weight.
- * Fan beam and ray tables take stream-ordered scratch (cudaMallocAsync) for
- * the image's transposed copy, which the walk reads where rays run closer to
- * the y axis; the sums are the same either way. */
+ * Fan beam and ray tables take stream-ordered scratch for the image's two
+ * copies (row-major and transposed, about 8 n^2 bytes), back projections for
+ * their 64-bit sums (8 bytes a pixel; cone beam 16 a voxel).  It comes from a
+ * pool of the library's own, which keeps up to 512 MB a device between calls
+ * and gives them back when the last plan is destroyed, when an allocation of
+ * the library's needs them, or through at_scratch_trim. */
 int at_forward(const at_plan *plan, const float *d_img, float *d_sino, void *stream);
 /* d_img = A^T d_sino; deterministic: each pixel is an exact integer sum of
  * fixed-point terms (no float atomics), so the result does not depend on
@@ -225,6 +228,10 @@ int at_back(const at_plan *plan, const float *d_sino, float *d_img, void *stream
 /* host-buffer forms: copy in, project, copy out, synchronise */
 int at_forward_host(const at_plan *plan, const float *h_img, float *h_sino);
 int at_back_host(const at_plan *plan, const float *h_sino, float *h_img);
+
+/* Gives back what the current device's scratch pool keeps and no call in flight
+ * uses, for programs that allocate beside the library. */
+int at_scratch_trim(void);
 
 /* ---- projection sets: several images through their plans in one launch ----
  * Batched form of at_forward / at_back (the reference projects one slice per

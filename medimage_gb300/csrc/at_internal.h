@@ -128,10 +128,18 @@ constexpr unsigned kSlabEmpty = 8u;       // no ray of the CTA crosses the image
 // Stream-ordered scratch of single calls, from a pool of the library's own that
 // keeps up to kScratchKept bytes between calls: the driver's default pool hands
 // everything back whenever the host waits for the GPU, and each call after a
-// wait then maps its scratch anew (190 us at any size).  The last plan to go
-// gives all of it back.  Freed with cudaFreeAsync.
+// wait then maps its scratch anew (190 us at any size).  What is kept is given
+// back when the last plan goes, when at_scratch_trim is called, and when an
+// allocation of the library's fails for want of it (dev_malloc).  Freed with
+// cudaFreeAsync.
 constexpr uint64_t kScratchKept = 512ull << 20;
 cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t st);
+void scratch_give_back();  // what no call in flight holds, of the current device
+cudaError_t dev_malloc_bytes(void **p, size_t bytes);
+template <typename T>
+cudaError_t dev_malloc(T **p, size_t bytes) {
+  return dev_malloc_bytes(reinterpret_cast<void **>(p), bytes);
+}
 struct ScratchUser {
   ScratchUser();
   ~ScratchUser();

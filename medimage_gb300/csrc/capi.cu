@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "../../include/goldnc.h"
+#include "alloc_retry.h"
 #include "solver.h"
 
 namespace medimg {
@@ -95,7 +96,20 @@ cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t st) {
     }
     pool = P.pool[dev];
   }
-  return cudaMallocFromPoolAsync(p, bytes, pool, st);
+  return alloc_or_give_back([&] { return cudaMallocFromPoolAsync(p, bytes, pool, st); }, scratch_give_back);
+}
+
+void scratch_give_back() {
+  cudaGetLastError();  // (the failed allocation's)
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= kMaxDevices) return;
+  ScratchPools &P = scratch_pools();
+  std::lock_guard<std::mutex> lock(P.mu);
+  if (P.pool[dev]) cudaMemPoolTrimTo(P.pool[dev], 0);
+}
+
+cudaError_t dev_malloc_bytes(void **p, size_t bytes) {
+  return alloc_or_give_back([&] { return cudaMalloc(p, bytes); }, scratch_give_back);
 }
 
 namespace {
@@ -470,9 +484,14 @@ AT_API int at_back_host(const at_plan *plan, const float *h_sino, float *h_img) 
 }
 
 // ---------------------------------------------------------------- device helpers
+AT_API int at_scratch_trim(void) {
+  scratch_give_back();
+  return AT_OK;
+}
+
 AT_API int at_dev_alloc(void **d_ptr, size_t bytes) {
   AT_CHECK_ARG(d_ptr, "at_dev_alloc: null argument");
-  AT_CUDA_TRY(cudaMalloc(d_ptr, bytes));
+  AT_CUDA_TRY(dev_malloc(d_ptr, bytes));
   return AT_OK;
 }
 AT_API int at_dev_free(void *d_ptr) {
@@ -689,9 +708,9 @@ struct GoldncContext {
     at_plan *p = nullptr;
     int rc = AT_OK;
     cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMalloc(&d, sizeof(double) * kGcPix);
-    if (e == cudaSuccess) e = cudaMalloc(&a, sizeof(float) * kGcPix);
-    if (e == cudaSuccess) e = cudaMalloc(&b, sizeof(float) * kGcPix);
+    if (e == cudaSuccess) e = dev_malloc(&d, sizeof(double) * kGcPix);
+    if (e == cudaSuccess) e = dev_malloc(&a, sizeof(float) * kGcPix);
+    if (e == cudaSuccess) e = dev_malloc(&b, sizeof(float) * kGcPix);
     if (e != cudaSuccess) rc = cuda_error(e, "GoldenC context set-up");
     if (!rc) rc = at_plan_create_goldnc(&p);
     if (rc) {

@@ -575,14 +575,14 @@ int build_cone_plan(Plan &p, cudaStream_t st) {
   p.cone_bp_views = cone_bp_views_per_chunk(g);
   std::vector<float2> trig(g.nproj);
   cone_trig(g, trig.data());
-  AT_CUDA_TRY(cudaMalloc(&p.cone_trig_d, sizeof(float2) * g.nproj));
+  AT_CUDA_TRY(dev_malloc(&p.cone_trig_d, sizeof(float2) * g.nproj));
   p.device_bytes += sizeof(float2) * g.nproj;
   AT_CUDA_TRY(cudaMemcpyAsync(p.cone_trig_d, trig.data(), sizeof(float2) * g.nproj, cudaMemcpyHostToDevice, st));
   ScanDev S;
   fill_scan_plan(S, p);
   unsigned long long *cnt = nullptr;
   const auto free_cnt = scope_exit([&] { cudaFree(cnt); });
-  AT_CUDA_TRY(cudaMalloc(&cnt, 3 * sizeof(unsigned long long)));
+  AT_CUDA_TRY(dev_malloc(&cnt, 3 * sizeof(unsigned long long)));
   AT_CUDA_TRY(cudaMemsetAsync(cnt, 0, 3 * sizeof(unsigned long long), st));
   cone_count_kernel<<<(unsigned)((p.rays + 255) / 256), 256, 0, st>>>(S, cnt, cnt + 1, (int *)(cnt + 2));
   AT_CUDA_TRY(cudaGetLastError());
@@ -606,9 +606,9 @@ int cone_trace_ray(const Plan &p, int64_t ray, int32_t *h_pix, float *h_w, int32
     cudaFree(wgt);
     cudaFree(cnt);
   });
-  AT_CUDA_TRY(cudaMalloc(&pix, sizeof(int) * dcap));
-  AT_CUDA_TRY(cudaMalloc(&wgt, sizeof(float) * dcap));
-  AT_CUDA_TRY(cudaMalloc(&cnt, sizeof(int)));
+  AT_CUDA_TRY(dev_malloc(&pix, sizeof(int) * dcap));
+  AT_CUDA_TRY(dev_malloc(&wgt, sizeof(float) * dcap));
+  AT_CUDA_TRY(dev_malloc(&cnt, sizeof(int)));
   cone_trace_one_kernel<<<1, 1>>>(S, ray, dcap, pix, wgt, cnt);
   AT_CUDA_TRY(cudaGetLastError());
   int n = 0;

@@ -401,7 +401,7 @@ cudaError_t launch_max(const unsigned *v, size_t n, unsigned *out, cudaStream_t 
 namespace {
 template <typename T>
 int dev_alloc(T **p, size_t count, int64_t &acct) {
-  cudaError_t e = cudaMalloc((void **)p, sizeof(T) * std::max<size_t>(count, 1));
+  cudaError_t e = dev_malloc((void **)p, sizeof(T) * std::max<size_t>(count, 1));
   if (e != cudaSuccess) return set_error(AT_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
   acct += (int64_t)(sizeof(T) * count);
   return AT_OK;
@@ -507,8 +507,8 @@ int build_fan_runs(Plan &p, cudaStream_t st) {
     cudaFree(cnt_d);
     cudaFree(cur_d);
   });
-  AT_CUDA_TRY(cudaMalloc(&cnt_d, sizeof(int) * ncell));
-  AT_CUDA_TRY(cudaMalloc(&cur_d, sizeof(unsigned long long)));
+  AT_CUDA_TRY(dev_malloc(&cnt_d, sizeof(int) * ncell));
+  AT_CUDA_TRY(dev_malloc(&cur_d, sizeof(unsigned long long)));
   AT_CUDA_TRY(cudaMemsetAsync(cnt_d, 0, sizeof(int) * ncell, st));
   AT_CUDA_TRY(cudaMemsetAsync(cur_d, 0, sizeof(unsigned long long), st));
   fan_runs_kernel<0><<<(nrays + tpb - 1) / tpb, tpb, 0, st>>>(p.n, p.nviews, p.ndets, p.nblocks_per_view, p.rays_d,
@@ -527,11 +527,11 @@ int build_fan_runs(Plan &p, cudaStream_t st) {
   if (tot >= (1ll << 31)) return set_error(AT_EINVAL, "plan: too many back-projection runs");
   off[ncell] = (int32_t)tot;
   p.nruns = tot;
-  AT_CUDA_TRY(cudaMalloc(&tmp_ent, sizeof(uint4) * std::max<int64_t>(tot, 1)));
-  AT_CUDA_TRY(cudaMalloc(&keys, sizeof(unsigned long long) * std::max<int64_t>(tot, 1)));
-  AT_CUDA_TRY(cudaMalloc(&keys_out, sizeof(unsigned long long) * std::max<int64_t>(tot, 1)));
-  AT_CUDA_TRY(cudaMalloc(&idx, sizeof(unsigned) * std::max<int64_t>(tot, 1)));
-  AT_CUDA_TRY(cudaMalloc(&idx_out, sizeof(unsigned) * std::max<int64_t>(tot, 1)));
+  AT_CUDA_TRY(dev_malloc(&tmp_ent, sizeof(uint4) * std::max<int64_t>(tot, 1)));
+  AT_CUDA_TRY(dev_malloc(&keys, sizeof(unsigned long long) * std::max<int64_t>(tot, 1)));
+  AT_CUDA_TRY(dev_malloc(&keys_out, sizeof(unsigned long long) * std::max<int64_t>(tot, 1)));
+  AT_CUDA_TRY(dev_malloc(&idx, sizeof(unsigned) * std::max<int64_t>(tot, 1)));
+  AT_CUDA_TRY(dev_malloc(&idx_out, sizeof(unsigned) * std::max<int64_t>(tot, 1)));
   fan_runs_kernel<1><<<(nrays + tpb - 1) / tpb, tpb, 0, st>>>(p.n, p.nviews, p.ndets, p.nblocks_per_view, p.rays_d,
                                                               p.bits_d, p.blk_word_d, p.ntiles_y, p.nvb, nullptr,
                                                               cur_d, tmp_ent, keys);
@@ -541,7 +541,7 @@ int build_fan_runs(Plan &p, cudaStream_t st) {
   // keys are unique (tile, view block, 63-nk, view, det): the sorted order is deterministic
   size_t temp_bytes = 0;
   AT_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, keys, keys_out, idx, idx_out, (int64_t)tot, 0, 64, st));
-  AT_CUDA_TRY(cudaMalloc(&temp, std::max<size_t>(temp_bytes, 1)));
+  AT_CUDA_TRY(dev_malloc(&temp, std::max<size_t>(temp_bytes, 1)));
   AT_CUDA_TRY(cub::DeviceRadixSort::SortPairs(temp, temp_bytes, keys, keys_out, idx, idx_out, (int64_t)tot, 0, 64, st));
   int rc;
   if ((rc = dev_alloc(&p.run_d, tot, p.device_bytes))) return rc;
@@ -564,7 +564,7 @@ int build_fan_runs(Plan &p, cudaStream_t st) {
   } else {
     const size_t cells = (size_t)p.n * p.n;
     unsigned *mx = nullptr;
-    AT_CUDA_TRY(cudaMalloc(&hits, sizeof(unsigned) * (cells + 1)));
+    AT_CUDA_TRY(dev_malloc(&hits, sizeof(unsigned) * (cells + 1)));
     mx = hits + cells;
     AT_CUDA_TRY(cudaMemsetAsync(mx, 0, sizeof(unsigned), st));
     for (int vb = 0; vb < p.nvb; vb++) {
@@ -600,9 +600,9 @@ int build_lines(Plan &p, const RaySource &R, cudaStream_t st) {
     cudaFree(first);
     cudaFree(line);
   });
-  AT_CUDA_TRY(cudaMalloc(&cnt_d, sizeof(int) * ((size_t)nrays + 1)));
-  AT_CUDA_TRY(cudaMalloc(&first, sizeof(LineCorr) * (size_t)nrays));
-  AT_CUDA_TRY(cudaMalloc(&line, sizeof(LineRay) * (size_t)nrays));
+  AT_CUDA_TRY(dev_malloc(&cnt_d, sizeof(int) * ((size_t)nrays + 1)));
+  AT_CUDA_TRY(dev_malloc(&first, sizeof(LineCorr) * (size_t)nrays));
+  AT_CUDA_TRY(dev_malloc(&line, sizeof(LineRay) * (size_t)nrays));
   line_rays_kernel<<<(nrays + tpb - 1) / tpb, tpb, 0, st>>>(R, line, first, cnt_d);
   AT_CUDA_TRY(cudaGetLastError());
   std::vector<int> off((size_t)nrays + 1);
@@ -648,13 +648,13 @@ int build_fan_plan(Plan &p, cudaStream_t st, const double *h_ends) {
   RaySource R{};
   R.g = g;
   if (h_ends) {
-    AT_CUDA_TRY(cudaMalloc(&tab_d, sizeof(double) * 4 * (size_t)nrays));
+    AT_CUDA_TRY(dev_malloc(&tab_d, sizeof(double) * 4 * (size_t)nrays));
     AT_CUDA_TRY(cudaMemcpyAsync(tab_d, h_ends, sizeof(double) * 4 * (size_t)nrays, cudaMemcpyHostToDevice, st));
     R.ends = tab_d;
   } else {
     std::vector<double> scos(nv), ssin(nv), dcos(nd), dsin(nd);
     fan_tables(g, scos.data(), ssin.data(), dcos.data(), dsin.data());
-    AT_CUDA_TRY(cudaMalloc(&tab_d, sizeof(double) * 2 * (nv + nd)));
+    AT_CUDA_TRY(dev_malloc(&tab_d, sizeof(double) * 2 * (nv + nd)));
     AT_CUDA_TRY(cudaMemcpyAsync(tab_d, scos.data(), sizeof(double) * nv, cudaMemcpyHostToDevice, st));
     AT_CUDA_TRY(cudaMemcpyAsync(tab_d + nv, ssin.data(), sizeof(double) * nv, cudaMemcpyHostToDevice, st));
     AT_CUDA_TRY(cudaMemcpyAsync(tab_d + 2 * nv, dcos.data(), sizeof(double) * nd, cudaMemcpyHostToDevice, st));
@@ -665,7 +665,7 @@ int build_fan_plan(Plan &p, cudaStream_t st, const double *h_ends) {
 
   if ((rc = dev_alloc(&p.rays_d, nrays, p.device_bytes))) return rc;
   int *off_d = nullptr;
-  AT_CUDA_TRY(cudaMalloc(&off_d, sizeof(int) * nrays));
+  AT_CUDA_TRY(dev_malloc(&off_d, sizeof(int) * nrays));
   const int tpb = 128;
   if (p.alpha_fp32)
     fan_count_kernel<float><<<(nrays + tpb - 1) / tpb, tpb, 0, st>>>(R, p.rays_d, off_d);
@@ -885,9 +885,9 @@ int build_goldnc_plan(Plan &p, cudaStream_t st) {
   }
   GcTrig *trig_d = nullptr;
   int *cnt_d = nullptr;
-  AT_CUDA_TRY(cudaMalloc(&trig_d, sizeof(GcTrig) * kGcAlphas));
+  AT_CUDA_TRY(dev_malloc(&trig_d, sizeof(GcTrig) * kGcAlphas));
   AT_CUDA_TRY(cudaMemcpyAsync(trig_d, trig.data(), sizeof(GcTrig) * kGcAlphas, cudaMemcpyHostToDevice, st));
-  AT_CUDA_TRY(cudaMalloc(&cnt_d, sizeof(int) * kGcWalks));
+  AT_CUDA_TRY(dev_malloc(&cnt_d, sizeof(int) * kGcWalks));
   gc_count_kernel<<<(kGcWalks + 127) / 128, 128, 0, st>>>(trig_d, cnt_d);
   AT_CUDA_TRY(cudaGetLastError());
   std::vector<int> cnt(kGcWalks);
@@ -909,7 +909,7 @@ int build_goldnc_plan(Plan &p, cudaStream_t st) {
   p.segments = tot;  // traced segments (each feeds up to 8 bins)
   int rc;
   int64_t *walk_off_d = nullptr;
-  AT_CUDA_TRY(cudaMalloc(&walk_off_d, sizeof(int64_t) * (kGcWalks + 1)));
+  AT_CUDA_TRY(dev_malloc(&walk_off_d, sizeof(int64_t) * (kGcWalks + 1)));
   AT_CUDA_TRY(cudaMemcpyAsync(walk_off_d, walk_off.data(), sizeof(int64_t) * (kGcWalks + 1),
                               cudaMemcpyHostToDevice, st));
   if ((rc = dev_alloc(&p.gc_seg_d, tot, p.device_bytes))) return rc;
@@ -921,7 +921,7 @@ int build_goldnc_plan(Plan &p, cudaStream_t st) {
 
   // transpose to per-pixel lists
   int *pcnt_d = nullptr;
-  AT_CUDA_TRY(cudaMalloc(&pcnt_d, sizeof(int) * kGcN * kGcN));
+  AT_CUDA_TRY(dev_malloc(&pcnt_d, sizeof(int) * kGcN * kGcN));
   AT_CUDA_TRY(cudaMemsetAsync(pcnt_d, 0, sizeof(int) * kGcN * kGcN, st));
   const int nb = (int)((tot + 255) / 256);
   gc_pix_count_kernel<<<nb, 256, 0, st>>>(p.gc_seg_d, tot, pcnt_d);

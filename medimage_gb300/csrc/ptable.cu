@@ -171,13 +171,13 @@ int build_pixel_table(Plan &p, int64_t max_bytes, cudaStream_t st) {
       cudaFree(w);
     }
   });
-  AT_CUDA_TRY(cudaMalloc(&meta, ncell * sizeof(uint32_t)));
-  AT_CUDA_TRY(cudaMalloc(&dend, ncell * sizeof(uint32_t)));
-  AT_CUDA_TRY(cudaMalloc(&voff, (size_t)nstreams * p.nviews * sizeof(uint32_t)));
-  AT_CUDA_TRY(cudaMalloc(&woff, (size_t)nstreams * (nch + 1) * sizeof(int64_t)));
-  AT_CUDA_TRY(cudaMalloc(&stotal, (size_t)nstreams * sizeof(int64_t)));
-  AT_CUDA_TRY(cudaMalloc(&base_d, (size_t)nstreams * sizeof(int64_t)));
-  AT_CUDA_TRY(cudaMalloc(&bad_d, sizeof(int)));
+  AT_CUDA_TRY(dev_malloc(&meta, ncell * sizeof(uint32_t)));
+  AT_CUDA_TRY(dev_malloc(&dend, ncell * sizeof(uint32_t)));
+  AT_CUDA_TRY(dev_malloc(&voff, (size_t)nstreams * p.nviews * sizeof(uint32_t)));
+  AT_CUDA_TRY(dev_malloc(&woff, (size_t)nstreams * (nch + 1) * sizeof(int64_t)));
+  AT_CUDA_TRY(dev_malloc(&stotal, (size_t)nstreams * sizeof(int64_t)));
+  AT_CUDA_TRY(dev_malloc(&base_d, (size_t)nstreams * sizeof(int64_t)));
+  AT_CUDA_TRY(dev_malloc(&bad_d, sizeof(int)));
   AT_CUDA_TRY(cudaMemsetAsync(meta, 0xff, ncell * sizeof(uint32_t), st));
   AT_CUDA_TRY(cudaMemsetAsync(dend, 0, ncell * sizeof(uint32_t), st));
   AT_CUDA_TRY(cudaMemsetAsync(bad_d, 0, sizeof(int), st));
@@ -203,7 +203,7 @@ int build_pixel_table(Plan &p, int64_t max_bytes, cudaStream_t st) {
   if (bytes > max_bytes) return AT_OK;
   cudaFree(dend);  // the largest temporary, before the weights are allocated
   dend = nullptr;
-  AT_CUDA_TRY(cudaMalloc(&w, (size_t)(entries + 4) * sizeof(float)));
+  AT_CUDA_TRY(dev_malloc(&w, (size_t)(entries + 4) * sizeof(float)));
   AT_CUDA_TRY(cudaMemsetAsync(w, 0, (size_t)(entries + 4) * sizeof(float), st));
   AT_CUDA_TRY(cudaMemcpyAsync(base_d, base.data(), sizeof(int64_t) * nstreams, cudaMemcpyHostToDevice, st));
   const int nwoff = nstreams * (nch + 1);

@@ -385,11 +385,11 @@ AT_API int at_rowaction_create(int32_t n, int32_t nproj, int32_t nray, at_rowact
   std::vector<float2> trig(nproj);
   for (int p = 0; p < nproj; p++) trig[p] = make_float2((float)std::sin(kMsPi / nproj * p), (float)std::cos(kMsPi / nproj * p));
   const int rays = nproj * nray;
-  AT_CUDA_TRY(cudaMalloc(&R->trig, sizeof(float2) * nproj));
+  AT_CUDA_TRY(dev_malloc(&R->trig, sizeof(float2) * nproj));
   AT_CUDA_TRY(cudaMemcpy(R->trig, trig.data(), sizeof(float2) * nproj, cudaMemcpyHostToDevice));
   int *cnt = nullptr;
   const auto free_cnt = scope_exit([&] { cudaFree(cnt); });
-  AT_CUDA_TRY(cudaMalloc(&cnt, sizeof(int) * rays));
+  AT_CUDA_TRY(dev_malloc(&cnt, sizeof(int) * rays));
   ra_count_kernel<<<(rays + 127) / 128, 128>>>(R->G, R->trig, cnt);
   AT_CUDA_TRY(cudaGetLastError());
   std::vector<int> h(rays);
@@ -400,9 +400,9 @@ AT_API int at_rowaction_create(int32_t n, int32_t nproj, int32_t nray, at_rowact
     off[r + 1] = off[r] + h[r];
   }
   R->segments = off[rays];
-  AT_CUDA_TRY(cudaMalloc(&R->off, sizeof(int64_t) * (rays + 1)));
-  AT_CUDA_TRY(cudaMalloc(&R->line, sizeof(int) * std::max<int64_t>(R->segments, 1)));
-  AT_CUDA_TRY(cudaMalloc(&R->weight, sizeof(float) * std::max<int64_t>(R->segments, 1)));
+  AT_CUDA_TRY(dev_malloc(&R->off, sizeof(int64_t) * (rays + 1)));
+  AT_CUDA_TRY(dev_malloc(&R->line, sizeof(int) * std::max<int64_t>(R->segments, 1)));
+  AT_CUDA_TRY(dev_malloc(&R->weight, sizeof(float) * std::max<int64_t>(R->segments, 1)));
   AT_CUDA_TRY(cudaMemcpy(R->off, off.data(), sizeof(int64_t) * (rays + 1), cudaMemcpyHostToDevice));
   ra_fill_kernel<<<(rays + 127) / 128, 128>>>(R->G, R->trig, R->off, R->line, R->weight);
   AT_CUDA_TRY(cudaGetLastError());

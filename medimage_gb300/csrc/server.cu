@@ -24,6 +24,7 @@
 #include <thread>
 #include <vector>
 
+#include "alloc_retry.h"
 #include "solver.h"
 
 namespace medimg {
@@ -123,7 +124,7 @@ struct Server {
       g->batch.params = prm;
       AT_CUDA_TRY(cudaStreamCreateWithFlags(&g->st, cudaStreamNonBlocking));
       AT_CUDA_TRY(cudaEventCreateWithFlags(&g->ev, cudaEventDisableTiming));
-      AT_CUDA_TRY(cudaMalloc(&g->psnr_scratch, psnr_scratch_bytes()));
+      AT_CUDA_TRY(dev_malloc(&g->psnr_scratch, psnr_scratch_bytes()));
     }
     *out = g.get();
     return AT_OK;
@@ -141,7 +142,7 @@ struct Server {
     if (rc) return rc;
     cudaStream_t gs = g->st;
     r->bytes = request_bytes(*r);
-    cudaError_t e = cudaMallocAsync(&r->mem, r->bytes, gs);
+    cudaError_t e = alloc_or_give_back([&] { return cudaMallocAsync(&r->mem, r->bytes, gs); }, scratch_give_back);
     if (e != cudaSuccess) return cuda_error(e, "server: state allocation");
     carve_scan(r->dev, *r->plan, rpt, (char *)r->mem);
     if (!r->ref.empty()) {

@@ -628,10 +628,10 @@ int build_slab_tables(Plan &p, int views, int rays, int rows, cudaStream_t st) {
     cudaFree(lo);
     cudaFree(hi);
   });
-  AT_CUDA_TRY(cudaMalloc(&flags, sizeof(unsigned) * ncta));
-  AT_CUDA_TRY(cudaMalloc(&fb, sizeof(unsigned) * ncta));
-  AT_CUDA_TRY(cudaMalloc(&lo, sizeof(int) * cells));
-  AT_CUDA_TRY(cudaMalloc(&hi, sizeof(int) * cells));
+  AT_CUDA_TRY(dev_malloc(&flags, sizeof(unsigned) * ncta));
+  AT_CUDA_TRY(dev_malloc(&fb, sizeof(unsigned) * ncta));
+  AT_CUDA_TRY(dev_malloc(&lo, sizeof(int) * cells));
+  AT_CUDA_TRY(dev_malloc(&hi, sizeof(int) * cells));
   AT_CUDA_TRY(cudaMemsetAsync(fb, 0, sizeof(unsigned) * ncta, st));
   AT_CUDA_TRY(cudaMemsetAsync(lo, 0x7f, sizeof(int) * cells, st));  // 0x7f7f7f7f: above any column
   AT_CUDA_TRY(cudaMemsetAsync(hi, 0x80, sizeof(int) * cells, st));  // 0x80808080: below any column
@@ -677,8 +677,8 @@ int build_slab_tables(Plan &p, int views, int rays, int rows, cudaStream_t st) {
   wbox = (wbox + 3) & ~3;
   if (wbox > 256) return AT_OK;  // wider than one TMA box: this shape does not fit
   SlabPlan &sp = p.slab;
-  AT_CUDA_TRY(cudaMalloc(&sp.cta_d, sizeof(uint4) * ncta));
-  AT_CUDA_TRY(cudaMalloc(&sp.wlo_d, sizeof(int16_t) * cells));
+  AT_CUDA_TRY(dev_malloc(&sp.cta_d, sizeof(uint4) * ncta));
+  AT_CUDA_TRY(dev_malloc(&sp.wlo_d, sizeof(int16_t) * cells));
   AT_CUDA_TRY(cudaMemcpyAsync(sp.cta_d, cta.data(), sizeof(uint4) * ncta, cudaMemcpyHostToDevice, st));
   AT_CUDA_TRY(cudaMemcpyAsync(sp.wlo_d, wlo.data(), sizeof(int16_t) * cells, cudaMemcpyHostToDevice, st));
   AT_CUDA_TRY(cudaStreamSynchronize(st));

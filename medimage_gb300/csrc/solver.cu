@@ -227,9 +227,9 @@ int Batch::set(const ScanDev *scans, int n, int kind_, int rpt_, cudaStream_t st
     prefix_d = nullptr;
     tmaps_d = nullptr;
     cap = std::max(n, 2 * cap);
-    AT_CUDA_TRY(cudaMalloc(&scans_d, sizeof(ScanDev) * cap));
-    AT_CUDA_TRY(cudaMalloc(&prefix_d, sizeof(int) * kFamilies * (cap + 1)));
-    AT_CUDA_TRY(cudaMalloc(&tmaps_d, sizeof(CUtensorMap) * cap));
+    AT_CUDA_TRY(dev_malloc(&scans_d, sizeof(ScanDev) * cap));
+    AT_CUDA_TRY(dev_malloc(&prefix_d, sizeof(int) * kFamilies * (cap + 1)));
+    AT_CUDA_TRY(dev_malloc(&tmaps_d, sizeof(CUtensorMap) * cap));
   }
   nscans = n;
   std::vector<ScanDev> sc(scans, scans + n);
@@ -362,14 +362,14 @@ int Batch::set(const ScanDev *scans, int n, int kind_, int rpt_, cudaStream_t st
         for (int u = pref[f * (n + 1) + s]; u < pref[f * (n + 1) + s + 1]; u++) order.push_back(u);
     }
     if (!queue_d) {
-      AT_CUDA_TRY(cudaMalloc(&queue_d, 2 * sizeof(unsigned)));
+      AT_CUDA_TRY(dev_malloc(&queue_d, 2 * sizeof(unsigned)));
       AT_CUDA_TRY(cudaMemsetAsync(queue_d, 0, 2 * sizeof(unsigned), st));
     }
     if (order.size() > order_cap) {
       cudaFree(order_d);
       order_d = nullptr;
       order_cap = std::max(order.size(), 2 * order_cap);
-      AT_CUDA_TRY(cudaMalloc(&order_d, sizeof(int) * order_cap));
+      AT_CUDA_TRY(dev_malloc(&order_d, sizeof(int) * order_cap));
     }
     if (!order.empty())
       AT_CUDA_TRY(cudaMemcpyAsync(order_d, order.data(), sizeof(int) * order.size(), cudaMemcpyHostToDevice, st));
@@ -594,7 +594,7 @@ int Solver::create(const std::vector<Plan *> &pl, const at_params &prm) {
   AT_CUDA_TRY(cudaStreamCreateWithFlags(&own_stream, cudaStreamNonBlocking));
   size_t total = 0;
   for (int s = 0; s < nscans; s++) total += scan_bytes(*pl[s], rpt);
-  if (cudaMalloc(&arena, total) != cudaSuccess) {
+  if (dev_malloc(&arena, total) != cudaSuccess) {
     cudaGetLastError();
     return set_error(AT_ENOMEM, "solver: device allocation of " + std::to_string(total) + " bytes failed");
   }
@@ -626,7 +626,7 @@ int ProjSet::create(const std::vector<Plan *> &pl) {
   const int n = (int)pl.size();
   size_t total = 256;
   for (auto *p : pl) total += bp_scratch_bytes(*p) + pack_bytes_of(*p);
-  if (cudaMalloc(&scratch, total) != cudaSuccess) {
+  if (dev_malloc(&scratch, total) != cudaSuccess) {
     cudaGetLastError();
     return set_error(AT_ENOMEM, "projection set: device allocation of " + std::to_string(total) + " bytes failed");
   }

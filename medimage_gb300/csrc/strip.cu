@@ -603,7 +603,7 @@ int strips_fit(const Plan &p, int ncr, cudaStream_t st, bool *fit) {
   const size_t cells = (size_t)p.n * p.n;
   unsigned *hits = nullptr;
   const auto free_hits = scope_exit([&] { cudaFree(hits); });
-  AT_CUDA_TRY(cudaMalloc(&hits, sizeof(unsigned) * (cells + 1)));
+  AT_CUDA_TRY(dev_malloc(&hits, sizeof(unsigned) * (cells + 1)));
   unsigned *const mx = hits + cells;
   AT_CUDA_TRY(cudaMemsetAsync(mx, 0, sizeof(unsigned), st));
   for (int v0 = 0; v0 < p.nviews; v0 += kBpViewBlock) {
@@ -640,9 +640,9 @@ int build_strips(Plan &p, const std::vector<int> &off, const std::vector<LineCor
   auto alloc = [&](auto **q, size_t count) {
     const size_t bytes = std::max<size_t>(16, count * sizeof(**q));
     p.device_bytes += (int64_t)bytes;
-    return cudaMalloc(q, bytes);
+    return dev_malloc(q, bytes);
   };
-  AT_CUDA_TRY(cudaMalloc(&count_d, sizeof(unsigned) * 2 * p.nviews));
+  AT_CUDA_TRY(dev_malloc(&count_d, sizeof(unsigned) * 2 * p.nviews));
   AT_CUDA_TRY(cudaMemsetAsync(count_d, 0, sizeof(unsigned) * 2 * p.nviews, st));
   AT_CUDA_TRY(alloc(&p.strip_rng_d, cells));
   strip_none_kernel<<<(unsigned)((cells + 255) / 256), 256, 0, st>>>(p.strip_rng_d, cells);

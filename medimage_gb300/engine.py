@@ -146,6 +146,7 @@ SIGNATURES = {
     "at_back": ([C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p], C.c_int),
     "at_forward_host": ([C.c_void_p, _fp, _fp], C.c_int),
     "at_back_host": ([C.c_void_p, _fp, _fp], C.c_int),
+    "at_scratch_trim": ([], C.c_int),
     "at_dev_alloc": ([C.POINTER(C.c_void_p), C.c_size_t], C.c_int),
     "at_dev_free": ([C.c_void_p], C.c_int),
     "at_memcpy_h2d": ([C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p], C.c_int),
