@@ -331,7 +331,8 @@ def run_ours(args):
     # The step's slices share one plan, so its projections run grouped (up to
     # four slices per walk of the plan): the grouped launches are timed through
     # a projection set over the step's slices, the single-slice kernels beside
-    # them.  A grouped launch's algorithmic bytes are its slices' sum.
+    # them.  Algorithmic bytes: each slice's input read once and its output
+    # written once (the rays' lines can be recomputed).
     G = B
     d_img = [torch.from_numpy(phantoms[b]).cuda() for b in range(G)]
     d_sino = [torch.from_numpy(sinos[b]).cuda() for b in range(G)]
@@ -341,17 +342,16 @@ def run_ours(args):
     ptr = lambda ts: [t.data_ptr() for t in ts]  # noqa: E731
     kern = {}
     cases = [
-        ("fan_fp_kernel", lambda: plan.forward_dev(d_img[0].data_ptr(), d_out_s[0].data_ptr(), st), 4 * S_seg + 4 * R),
-        ("fan_bp_kernel", lambda: plan.back_dev(d_sino[0].data_ptr(), d_out_i[0].data_ptr(), st), 4 * S_seg + 4 * P)]
+        ("line_fp_kernel", lambda: plan.forward_dev(d_img[0].data_ptr(), d_out_s[0].data_ptr(), st), 4 * P + 4 * R),
+        ("strip_bp_kernel", lambda: plan.back_dev(d_sino[0].data_ptr(), d_out_i[0].data_ptr(), st), 4 * P + 4 * R)]
     if G > 1:
         cases += [
-            ("fan_fp_kernel<group>", lambda: pset.forward_dev(ptr(d_img), ptr(d_out_s), st), G * (4 * S_seg + 4 * R)),
-            ("fan_bp_group_kernel", lambda: pset.back_dev(ptr(d_sino), ptr(d_out_i), st), G * (4 * S_seg + 4 * P))]
+            ("line_fp_kernel (groups)", lambda: pset.forward_dev(ptr(d_img), ptr(d_out_s), st), G * (4 * P + 4 * R)),
+            ("strip_bp_kernel (groups)", lambda: pset.back_dev(ptr(d_sino), ptr(d_out_i), st), G * (4 * P + 4 * R))]
     for name, fn, nbytes in cases:
         for _ in range(3):
             fn()
-        # L2 flushed before every timed launch (as in the step, where the back
-        # projector's run list evicts the forward projector's plan)
+        # L2 flushed before every timed launch
         reps = 20
         evs = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)) for _ in range(reps)]
         for e0, e1 in evs:
@@ -378,8 +378,8 @@ def run_ours(args):
     prof = profile_counters(dom)
     traffic = prof.get("dram_bytes")
     if traffic is not None and "group" in dom:
-        # captured on one group of four slices; each group of a launch streams
-        # the plan once, so DRAM traffic scales with the groups in the launch
+        # captured on one group of four slices; each group of a launch reads the
+        # rays' lines once, so DRAM traffic scales with the groups in the launch
         traffic = int(traffic * ((G + 3) // 4))
     dram_frac = None if traffic is None else traffic / (kern[dom]["ms"] / 1e3) / 1e9 / peak
     gsegs = S_seg * (fp_calls + bp_calls) * slices / (ms / 1e3) / 1e9
@@ -419,9 +419,9 @@ def run_ours(args):
                          "dram_frac": None if dram_frac is None else round(dram_frac, 4),
                          "limiter": {k: prof[k] for k in ("unit", "throughput_pct", "sectors_per_request",
                                                           "issue_active_pct", "source") if k in prof},
-                         "note": ("achieved = algorithmic bytes (4 S + 4 R per slice) / CUDA-event time: an "
-                                  "effective gather rate, not DRAM traffic.  The images, sinograms and most of "
-                                  "the plan stay in the 129 MB L2, so the kernel is bound by the SM's load path "
+                         "note": ("achieved = algorithmic bytes (4 P + 4 R per slice: input read, output written "
+                                  "once) / CUDA-event time.  The kernel gathers (or adds to) some 2 n pixels a ray "
+                                  "from copies that stay in the 129 MB L2, so it is bound by the SM's load path "
                                   "(the 'limiter' unit, from ncu), and its DRAM traffic ('traffic', ncu) is "
                                   "dram_frac of the measured HBM peak") if prof.get("bound", "hbm") != "hbm"
                          else None,

@@ -112,13 +112,16 @@ typedef struct at_plan_stats {
     int64_t offgrid;       /* segments the reference traces off the pixel grid */
     int64_t device_bytes;  /* plan memory in HBM                               */
     int32_t max_segments;  /* longest ray                                      */
-    int32_t fp_rays_per_thread; /* forward-projector variant the autotuner chose */
-    int64_t bp_runs;       /* (ray, 16x16 tile) runs the back projector walks   */
+    int32_t fp_rays_per_thread; /* rays per thread of the walk by decision bits, as
+                                 * the autotuner chose; 1 where rays are lines  */
+    int64_t bp_runs;       /* (ray, 16x16 tile) runs of the traversal            */
     int32_t nz;            /* image slices (1 for 2D plans)                      */
-    /* forward projector through shared-memory slabs (fan / ray plans), when the
-     * autotuner chose it over the L1 walk: CTA shape (views x adjacent
-     * detectors), rows per slab, staged columns per slab, and the CTAs that
-     * gather through L1 because a ray leaves the grid; all 0 otherwise */
+    /* forward projector through shared-memory slabs (fan / ray plans), where
+     * at_plan_set_forward_variant pinned it, or the autotuner chose it over the
+     * walk by decision bits (plans whose rays are not walked as lines): CTA
+     * shape (views x adjacent detectors), rows per slab, staged columns per
+     * slab, and the CTAs that gather through L1 because a ray leaves the grid
+     * or runs against the others; all 0 otherwise */
     int32_t slab_views, slab_rays, slab_rows, slab_wbox, slab_fallback_ctas;
     /* back projection from the pixel table (at_plan_set_back_variant): the
      * launches that use it (bit0 single scans, bit1 groups of scans sharing
@@ -155,9 +158,11 @@ int at_plan_create_cone(const at_cone_geometry *geom, at_plan **out);
  * (msbeam/CPU_OpenMP/src/proj.c:53-65).  The table is copied. */
 int at_plan_create_rays(int32_t n, double pixel_mm, int32_t nviews, int32_t ndets, const double *h_endpoints,
                         at_plan **out);
-/* Pins the forward projector of a fan-beam or ray-table plan, in place of the
- * autotuner's choice (results are bitwise the same for every variant):
- * views = rays = rows = 0 selects the walk that gathers through L1;
+/* Pins the forward projector of a fan-beam or ray-table plan (results are
+ * bitwise the same for every variant).  By default rays are walked as lines,
+ * gathering through L1; for plans traced in FP32, and ray tables with many rays
+ * that end inside the grid, the plan times the walk by decision bits and slabs
+ * and keeps the faster.  views = rays = rows = 0 selects the walk through L1;
  * otherwise the slab projector with CTAs of `views` consecutive views x
  * `rays` adjacent detectors (rays divides 128, views * rays <= 512) and slabs
  * of `rows` image rows.  AT_EINVAL if the shape does not fit this plan (the
@@ -198,7 +203,8 @@ void at_plan_destroy(at_plan *plan);
  * groups) made after the call, fan-beam and ray-table plans: 0 = one CTA per
  * work unit (the default), 1 = persistent, a grid of the resident CTAs pulling
  * (scan, view, ray block) and (scan, pixel tile) units from a queue, the
- * costlier scans' units first.  Results are bitwise the same.  On GB300 the
+ * costlier scans' units first; back projections along lines and slabs keep one
+ * CTA per work unit in either form.  Results are bitwise the same.  On GB300 the
  * persistent form measured 8-9 % slower (C2, 16 slices; C3): a CTA's finished
  * warps wait at each unit's end while the hardware scheduler would start a new
  * CTA beside them.  The reference has no batched form (its only GPU code,

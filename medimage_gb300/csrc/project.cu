@@ -413,10 +413,10 @@ __global__ void __launch_bounds__(128) fan_fp_queue_kernel(const Launch L) {
 // lanes of the segment walk, at equal step counts but in a dozen different
 // rows, touch about ten.  A row costs two gathers (current and next column; a
 // predicated second one measured slower) and no decision bits.
-// Bound: instruction issue and load latency for one member (58 % issue, 44 %
-// L1 at C2), the L1 data path for four (84 %: 2 x 16 bytes a row and lane).
-// C2, the image's copies included: one slice 243 -> 130 us, eight slices
-// 812 -> 560 us; error against 64 bits 2.2e-7 -> 1.3e-7.
+// Bound: instruction issue and load latency for one member (73 % issue, 50 %
+// L1 at C2), the L1 data path for four (78 %: 2 x 16 bytes a row and lane).
+// C2, the image's copies included: one slice 243 -> 126 us, eight slices
+// 812 -> 546 us; error against 64 bits 2.1e-7 -> 1.2e-7.
 template <int G, int kBatch = 2>
 __device__ __forceinline__ void line_fp_body(const Launch &L, const int unit) {
   using T = typename Elem<G>::T;
@@ -448,7 +448,8 @@ __device__ __forceinline__ void line_fp_body(const Launch &L, const int unit) {
   w.load(ray);
   const bool swap = (ray.flags & kLineSwap) != 0, down = (ray.flags & kLineDown) != 0, none = w.empty();
   // The lane's copy and its rows in walk order: element row0 + step * stride +
-  // (padded) column.  A lane without a line reads the zeros at element 0.
+  // (padded) column.  A lane without a line never crosses: it reads the zeros at
+  // element 0.
   const int c0 = none ? -kLinePad : line_c0(ray, n, line_pitch(n));
   const int row0 = none ? 0 : (swap ? n * pitch : 0) + (down ? (n - 1) * pitch : 0);
   const int stride = none ? 0 : down ? -pitch : pitch;
@@ -1246,8 +1247,6 @@ int bp_split_for(int tiles, int nvb) {
 int pix_ctas(const ScanDev &S) { return ((S.n + kPixRows - 1) / kPixRows) * ((S.n + 31) / 32) * S.nz; }
 
 // the forms of a launch's scans (Launch::forms)
-int line_ctas(const ScanDev &S, int threads);
-
 int launch_forms(const Launch &L) { return L.scans ? L.forms : L.single.line ? 2 : 1; }
 
 // Fan-beam / ray-table scans: the walk along lines (the scans' pack buffers
@@ -1447,8 +1446,9 @@ int launch_fp_tr(const Launch &L, const Launch &Lpix, int rpt, int nctas, int pi
 int launch_bp_group(const Launch &L, const Launch &Lsino, const Launch &Lsmall, const Launch &Lpix, int nctas,
                     int sino_nctas, int small_nctas, int pix_nctas, cudaStream_t st) {
   int n = 2;
-  Launch La = L;  // the max |r| pass: one CTA per part, never queued
+  Launch La = L;  // the max |r| pass: one CTA per part, never queued; the sums are zero
   La.queue = nullptr;
+  La.flag = 0;
   launch_dependent(sino_absmax_kernel, L.nscans * kBpMaxParts, 256, 0, st, La);
   launch_dependent(fp_pack_kernel, sino_nctas, 256, 0, st, Lsino, 1);
   static int resg[3] = {0, 0, 0}, ress[3] = {0, 0, 0};

@@ -16,11 +16,14 @@
 // stream (288 MB at 512^2, 720 x 888), no decision bits, and the lanes of a
 // warp, neighbouring rays in the same row, add side by side instead of in a
 // dozen rows of a small tile (two wavefronts an add for almost four).  512^2,
-// 720 x 888: one slice 287 -> 180 us, sixteen slices 2.51 -> 1.72 ms; 1024^2,
-// 1440 x 1536: 1.70 -> 1.02 ms; error against 64 bits 5.9e-7 -> 2e-7 (a
+// 720 x 888: one slice 287 -> 181 us, sixteen slices 2.51 -> 1.73 ms; 1024^2,
+// 1440 x 1536: 1.70 -> 1.02 ms; error against 64 bits 5.9e-7 -> 1.9e-7 (a
 // crossing is rounded as a row number, not as a distance from the source).
-// Bound: the L1 data pipe (88 % of its wavefronts while CTAs run; two an add,
-// because 32 neighbouring rays cover either more or fewer than 32 columns).
+// The forward walk takes a line up every 32 rows, the strips every 16, so that
+// the two sides' weights agree to the rounding of a crossing.
+// Bound: the L1 data pipe (78 % while CTAs run, 93 % with four members; two
+// wavefronts an add, because 32 neighbouring rays cover either more or fewer
+// than 32 columns), then issue (77 %, 72 %).
 // Measured and left: 16-row strips for one member (more loads of rays), the
 // gather by pixel of every ray that can cross it (340 us one slice, 571 us four
 // slices against 190 and 552: address arithmetic and 16-byte shared loads).

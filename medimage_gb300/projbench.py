@@ -1,11 +1,13 @@
 """Time the forward and back projectors alone on one workload geometry.
 
     python -m medimage_gb300.projbench [--config c1|c2|c4] [--n N] [--reps N] [--which fp,bp] [--group G]
-                                       [--variant l1|views,rays,rows] [--bp runs|table]
+                                       [--variant l1|views,rays,rows] [--bp lines|runs|table]
 
 Prints one JSON line per projector: average launch time (CUDA events on the
-launching stream around each launch, L2 flushed before each unless --warm), algorithmic bytes per launch (forward 4 S + 4 R, back
-4 S + 4 P; S segments, R rays, P pixels or voxels) and the resulting GB/s.
+launching stream around each launch, L2 flushed before each unless --warm),
+algorithmic bytes per launch (input read and output written once: 4 P + 4 R
+for R rays and P pixels; for the cone beam, whose segments are gathered one by
+one, forward 4 S + 4 R and back 4 S + 4 P) and the resulting GB/s.
 Used as the command under the profiler as well.  c4 is the 512^3 cone beam
 (--n shrinks the volume, same field of view).  --group G (2D) projects G
 images of the plan together through a projection set, the grouped kernels
@@ -33,10 +35,10 @@ def main() -> None:
     ap.add_argument("--warm", action="store_true", help="no L2 flush between timed launches")
     ap.add_argument("--variant", default="",
                     help="forward projector of 2D plans: 'l1', or views,rays,rows of the slab projector "
-                         "(default: the autotuner's choice)")
-    ap.add_argument("--bp", default="", choices=["", "runs", "table"],
-                    help="back projector of 2D plans: walk tile runs, or gather from the pixel table "
                          "(default: the plan's choice)")
+    ap.add_argument("--bp", default="lines", choices=["lines", "runs", "table"],
+                    help="back projector of 2D plans: along lines (the plan's default), tile runs, or gathered "
+                         "from the pixel table")
     args = ap.parse_args()
     if args.config == "c4":
         spec = configs.c4(n=args.n, nz=args.n)
@@ -49,10 +51,11 @@ def main() -> None:
         if args.variant:
             plan.set_forward_variant(*([0, 0, 0] if args.variant == "l1" else
                                        [int(x) for x in args.variant.split(",")]))
-        if args.bp:
+        if args.bp != "lines":
             plan.set_back_variant(3 if args.bp == "table" else 0)
         img = phantom.ellipse_phantom(plan.n, seed=spec.seed, n_random=spec.n_random)
-        names = ("fan_fp_kernel", "fan_bp_kernel")
+        names = ("fan_fp_slab_kernel" if plan.stats["slab_views"] else "line_fp_kernel",
+                 "strip_bp_kernel" if plan.back_variant < 0 else "fan_bp_kernel")
     L = engine.lib()
     st = C.c_void_p()
     engine._check("at_stream_create", L.at_stream_create(C.byref(st)))
@@ -69,19 +72,20 @@ def main() -> None:
 
     ts = torch.cuda.ExternalStream(st.value)
     S, R, P = plan.stats["segments"], plan.stats["rays"], int(np.prod(plan.img_shape))
+    cone = args.config == "c4"
     jobs = {
-        "fp": (names[0], lambda: plan.forward_dev(bufs["img"], bufs["sino_out"], st.value), 4 * S + 4 * R),
-        "bp": (names[1], lambda: plan.back_dev(bufs["sino"], bufs["img_out"], st.value), 4 * S + 4 * P),
+        "fp": (names[0], lambda: plan.forward_dev(bufs["img"], bufs["sino_out"], st.value), 4 * (S if cone else P) + 4 * R),
+        "bp": (names[1], lambda: plan.back_dev(bufs["sino"], bufs["img_out"], st.value), 4 * (S if cone else R) + 4 * P),
     }
     pset = None
     if G > 1:
         pset = engine.ProjSet([plan] * G)
         sel = lambda key: [bufs[key if g == 0 else f"{key}{g}"] for g in range(G)]  # noqa: E731
         jobs = {
-            "fp": ("fan_fp_kernel<group>", lambda: pset.forward_dev(sel("img"), sel("sino_out"), st.value),
-                   G * (4 * S + 4 * R)),
-            "bp": ("fan_bp_group_kernel", lambda: pset.back_dev(sel("sino"), sel("img_out"), st.value),
-                   G * (4 * S + 4 * P)),
+            "fp": (names[0] + " (groups)", lambda: pset.forward_dev(sel("img"), sel("sino_out"), st.value),
+                   G * (4 * P + 4 * R)),
+            "bp": (names[1] + " (groups)", lambda: pset.back_dev(sel("sino"), sel("img_out"), st.value),
+                   G * (4 * P + 4 * R)),
         }
     flush = torch.empty(256 * 1024 * 1024 // 4, dtype=torch.float32, device="cuda")
     for key in args.which.split(","):
